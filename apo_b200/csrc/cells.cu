@@ -55,12 +55,16 @@ namespace apo2
     // -----------------------------------------------------------------------------------
     // The cell of one warp, in shared memory
     // -----------------------------------------------------------------------------------
+    // Fp32: the filtered form's instantiation (apo2_options.precision).
+    template<bool Fp32>
     struct WarpCell
     {
         uint4 * v;       // (j, k, l, type | status << 8), capacity kVertexSlots
         double4 * pos;   // solved position of v[*]
         uint4 * e;       // (j, k, vertex count, status | validated << 8), capacity kEdgeSlots
+        uint32_t * u;    // distinct sites of e[*] (the cell's neighbours), capacity kSiteSlots
         uint32_t vn, en; // warp-uniform sizes
+        uint32_t un;     // neighbours in u, or kNone: more than kSiteSlots, e[*] is scanned instead
         mutable FilterTally tally; // this lane's FP32-filter counts
     };
 
@@ -69,24 +73,112 @@ namespace apo2
     __device__ __forceinline__ uint32_t estatus( uint4 r ) { return r.w & 0xffu; }
 
 
-    // Default validation predicate of the cell update (topology_update.inl:578-592): no site
-    // of the cell's edges other than skip1 / skip2 intersects `sphere`. Warp-collective;
-    // returns the warp-wide result. The reference tests every edge; the loop stops once a
-    // conflict is known, which does not change the result.
-    __device__ __forceinline__ bool edges_clear( const CellContext & c, const WarpCell & w, double4 sphere, uint32_t skip1,
-                                                 uint32_t skip2 )
+    // The sites the emptiness and known-neighbour tests range over, those of the cell's edges, as a
+    // sequence. The neighbour list holds each once (an edge list names every neighbour about six
+    // times); a cell with more neighbours than slots goes by its edges.
+    struct SiteSequence
     {
-        bool ok = true;
+        const uint32_t * words;
+        uint32_t         count, shift; // shift 0: a list of ids; 1: two ids at the front of 16-byte records
+        __device__ __forceinline__ uint32_t operator[]( uint32_t q ) const
+        {
+            return words[ ( ( q >> shift ) << ( 2 * shift ) ) + ( q & shift ) ];
+        }
+    };
+    template<class W>
+    __device__ __forceinline__ SiteSequence sites_of( const W & w )
+    {
+        if ( w.un != kNone )
+            return { w.u, w.un, 0u };
+        return { reinterpret_cast<const uint32_t *>( w.e ), 2u * w.en, 1u };
+    }
+
+    // The neighbour list from the edges alone. Warp-collective.
+    template<class W>
+    __device__ __forceinline__ void list_sites( W & w )
+    {
+        const uint32_t lane = lane_id();
+        uint32_t       n    = 0;
         for ( uint32_t base = 0; base < w.en; base += 32 )
         {
-            const uint32_t e = base + lane_id();
-            if ( e < w.en )
+            const bool  in = base + lane < w.en;
+            const uint4 r  = in ? w.e[ base + lane ] : make_uint4( kNone, kNone, 0, 0 );
+#pragma unroll 1
+            for ( uint32_t s = 0; s < 2; s++ )
             {
-                const uint4 r = w.e[ e ];
-                if ( r.x != skip1 && r.x != skip2 )
-                    ok = ok && !site_conflict( c, r.x, sphere, w.tally );
-                if ( r.y != skip1 && r.y != skip2 )
-                    ok = ok && !site_conflict( c, r.y, sphere, w.tally );
+                const uint32_t id    = s ? r.y : r.x;
+                const uint32_t peers = __match_any_sync( kFull, id );
+                bool           add   = in && lane == __ffs( peers ) - 1;
+                for ( uint32_t q = 0; q < n; q++ )
+                    add = add && w.u[ q ] != id;
+                const uint32_t bal = __ballot_sync( kFull, add );
+                if ( n + __popc( bal ) > kSiteSlots )
+                {
+                    w.un = kNone;
+                    return;
+                }
+                if ( add )
+                    w.u[ n + __popc( bal & ( ( 1u << lane ) - 1u ) ) ] = id;
+                n += __popc( bal );
+                __syncwarp();
+            }
+        }
+        w.un = n;
+    }
+
+    // The neighbour list after an update by site j: j and the former neighbours that still have an
+    // edge. Warp-collective.
+    template<class W>
+    __device__ __forceinline__ void relist_sites( W & w, uint32_t j )
+    {
+        const uint32_t lane = lane_id();
+        if ( w.un >= kSiteSlots ) // no list, or none to spare for j
+        {
+            list_sites( w );
+            return;
+        }
+        const uint32_t had  = w.un;
+        uint32_t       kept = 0;
+#pragma unroll 1
+        for ( uint32_t base = 0; base <= had; base += 32 )
+        {
+            const uint32_t q  = base + lane;
+            const uint32_t id = q < had ? w.u[ q ] : ( q == had ? j : kNone );
+            bool           keep = false;
+#pragma unroll 4
+            for ( uint32_t e = 0; e < w.en; e++ )
+            {
+                const uint2 r = *reinterpret_cast<const uint2 *>( &w.e[ e ] );
+                keep          = keep || r.x == id || r.y == id;
+            }
+            const uint32_t bal = __ballot_sync( kFull, keep );
+            if ( keep )
+                w.u[ kept + __popc( bal & ( ( 1u << lane ) - 1u ) ) ] = id;
+            kept += __popc( bal );
+            __syncwarp();
+        }
+        w.un = kept;
+    }
+
+    // Default validation predicate of the cell update (topology_update.inl:578-592): no site
+    // of the cell's edges other than skip1 / skip2 intersects `sphere`. Warp-collective, one sphere;
+    // returns the warp-wide result. The loop stops once a conflict is known, which does not
+    // change the result.
+    template<bool Fp32>
+    __device__ __forceinline__ bool edges_clear( const CellContext & c, const WarpCell<Fp32> & w, double4 sphere, uint32_t skip1,
+                                                 uint32_t skip2 )
+    {
+        bool               ok    = true;
+        const SiteSequence sites = sites_of( w );
+#pragma unroll 1
+        for ( uint32_t base = 0; base < sites.count; base += 32 )
+        {
+            const uint32_t q = base + lane_id();
+            if ( q < sites.count )
+            {
+                const uint32_t id = sites[ q ];
+                if ( id != skip1 && id != skip2 )
+                    ok = !site_conflict<Fp32>( c, id, sphere, w.tally );
             }
             if ( !__all_sync( kFull, ok ) )
                 return false;
@@ -94,50 +186,68 @@ namespace apo2
         return true;
     }
 
-#ifndef APO2_LANE_CLEAR_EDGES
-#define APO2_LANE_CLEAR_EDGES 8
-#endif
-    // cells with at most this many edges check new roots lane by lane in update_cell
-    constexpr uint32_t kLaneClearEdges = APO2_LANE_CLEAR_EDGES;
-
-    // Lane-local forms of is_known / edges_clear (same predicates, one lane scanning all edges).
-    __device__ __forceinline__ bool known_by_lane( const WarpCell & w, uint32_t id )
+    // The same predicate for up to two spheres per lane at once (bits of `open`): every lane goes
+    // through the neighbours together, so a neighbour is loaded once for all lanes' spheres and the
+    // tests of one lane do not depend on one another. Returns the bits that stay clear. (Checking
+    // one lane's sphere at a time with a neighbour per lane, as the reference does, spent 65 to
+    // 80 % of the update on votes and shuffles around few tests: cells have 8 to 13 neighbours
+    // while 20 to 50 spheres are checked per update.)
+    template<bool Fp32>
+    __device__ __forceinline__ uint32_t spheres_clear( const CellContext & c, const WarpCell<Fp32> & w, double4 x0, double4 x1,
+                                                       uint32_t open, uint32_t skip1, uint32_t skip2 )
     {
-        for ( uint32_t e = 0; e < w.en; e++ )
+        const SiteSequence sites = sites_of( w );
+#pragma unroll 1
+        for ( uint32_t q = 0; q < sites.count; q++ )
         {
-            const uint4 r = w.e[ e ];
-            if ( r.x == id || r.y == id )
-                return true;
+            if ( !__any_sync( kFull, open ) )
+                break;
+            const uint32_t id = sites[ q ];
+            if ( id != skip1 && id != skip2 )
+            {
+                if ( ( open & 1u ) && site_conflict<Fp32>( c, id, x0, w.tally ) )
+                    open &= ~1u;
+                if ( ( open & 2u ) && site_conflict<Fp32>( c, id, x1, w.tally ) )
+                    open &= ~2u;
+            }
         }
+        return open;
+    }
+
+    // Lane-local forms of is_known / edges_clear (same predicates, one lane scanning all sites).
+    template<class W>
+    __device__ __forceinline__ bool known_by_lane( const W & w, uint32_t id )
+    {
+        const SiteSequence sites = sites_of( w );
+        for ( uint32_t q = 0; q < sites.count; q++ )
+            if ( sites[ q ] == id )
+                return true;
         return false;
     }
-    __device__ __forceinline__ bool clear_by_lane( const CellContext & c, const WarpCell & w, double4 sphere, uint32_t skip1,
+    template<bool Fp32>
+    __device__ __forceinline__ bool clear_by_lane( const CellContext & c, const WarpCell<Fp32> & w, double4 sphere, uint32_t skip1,
                                                    uint32_t skip2 )
     {
-        for ( uint32_t e = 0; e < w.en; e++ )
+        const SiteSequence sites = sites_of( w );
+        for ( uint32_t q = 0; q < sites.count; q++ )
         {
-            const uint4 r = w.e[ e ];
-            if ( r.x != skip1 && r.x != skip2 && site_conflict( c, r.x, sphere, w.tally ) )
-                return false;
-            if ( r.y != skip1 && r.y != skip2 && site_conflict( c, r.y, sphere, w.tally ) )
+            const uint32_t id = sites[ q ];
+            if ( id != skip1 && id != skip2 && site_conflict<Fp32>( c, id, sphere, w.tally ) )
                 return false;
         }
         return true;
     }
 
     // Is `id` already a neighbour of the cell (one of its edges' sites)? Warp-collective.
-    __device__ __forceinline__ bool is_known( const WarpCell & w, uint32_t id )
+    template<class W>
+    __device__ __forceinline__ bool is_known( const W & w, uint32_t id )
     {
-        for ( uint32_t base = 0; base < w.en; base += 32 )
+        const SiteSequence sites = sites_of( w );
+#pragma unroll 1
+        for ( uint32_t base = 0; base < sites.count; base += 32 )
         {
-            const uint32_t e   = base + lane_id();
-            bool           hit = false;
-            if ( e < w.en )
-            {
-                const uint4 r = w.e[ e ];
-                hit           = r.x == id || r.y == id;
-            }
-            if ( __any_sync( kFull, hit ) )
+            const uint32_t q = base + lane_id();
+            if ( __any_sync( kFull, q < sites.count && sites[ q ] == id ) )
                 return true;
         }
         return false;
@@ -153,65 +263,130 @@ namespace apo2
 
     struct NewEdges
     {
-        uint32_t slot[ 2 ];
+        uint32_t slot[ 2 ]; // candidate t in slot[t / 32] of lane t % 32
         uint32_t count; // warp-uniform
-        __device__ __forceinline__ void push( uint32_t k, bool two, bool closed, uint32_t & err )
+        __device__ __forceinline__ void push( uint32_t packed, uint32_t & err )
         {
             if ( count < kMaxNewEdges )
             {
-                if ( lane_id() == count / 2 )
-                    slot[ count & 1 ] = pack_edge( k, two, closed );
+                if ( lane_id() == ( count & 31u ) )
+                    slot[ count >> 5 ] = packed;
             }
             else
                 err |= kErrNewEdgeCap;
             count++;
         }
-        __device__ __forceinline__ bool contains( uint32_t k ) const
-        {
-            const bool hit = ( slot[ 0 ] >> 2 ) == k || ( slot[ 1 ] >> 2 ) == k;
-            return __any_sync( kFull, hit );
-        }
     };
 
-    // Ascending bitonic sort of the 64 packed candidates (element 2*lane + s in slot[s]).
+    // Ascending bitonic sort of the 64 packed candidates; element 2*lane + s ends in slot[s].
     __device__ __forceinline__ void sort64( uint32_t ( &a )[ 2 ] )
     {
         const uint32_t lane = lane_id();
-#pragma unroll
+#pragma unroll 1
         for ( uint32_t size = 2; size <= 64; size <<= 1 )
         {
-#pragma unroll
-            for ( uint32_t stride = size >> 1; stride > 0; stride >>= 1 )
+#pragma unroll 1
+            for ( uint32_t stride = size >> 1; stride > 1; stride >>= 1 )
             {
-                if ( stride == 1 )
-                {
-                    const bool up = ( ( 2 * lane ) & size ) == 0;
-                    if ( ( a[ 0 ] > a[ 1 ] ) == up )
-                    {
-                        const uint32_t t = a[ 0 ];
-                        a[ 0 ]           = a[ 1 ];
-                        a[ 1 ]           = t;
-                    }
-                }
-                else
-                {
 #pragma unroll
-                    for ( uint32_t s = 0; s < 2; s++ )
-                    {
-                        const uint32_t f     = 2 * lane + s;
-                        const uint32_t other = __shfl_xor_sync( kFull, a[ s ], stride >> 1 );
-                        const bool     lower = ( f & stride ) == 0;
-                        const bool     up    = ( f & size ) == 0;
-                        a[ s ]               = ( lower == up ) ? min( a[ s ], other ) : max( a[ s ], other );
-                    }
+                for ( uint32_t s = 0; s < 2; s++ )
+                {
+                    const uint32_t f     = 2 * lane + s;
+                    const uint32_t other = __shfl_xor_sync( kFull, a[ s ], stride >> 1 );
+                    const bool     lower = ( f & stride ) == 0;
+                    const bool     up    = ( f & size ) == 0;
+                    a[ s ]               = ( lower == up ) ? min( a[ s ], other ) : max( a[ s ], other );
                 }
+            }
+            const bool up = ( ( 2 * lane ) & size ) == 0;
+            if ( ( a[ 0 ] > a[ 1 ] ) == up )
+            {
+                const uint32_t t = a[ 0 ];
+                a[ 0 ]           = a[ 1 ];
+                a[ 1 ]           = t;
             }
         }
     }
 
+    // The new edges of an update by site j: one per distinct candidate site, ascending, with the
+    // number of its candidates (new vertices), appended to w.e (topology_update.inl:435-515). Returns
+    // how many there are. More than 32 candidates are sorted; up to 32, nearly always, each lane
+    // holds one and finds its group by a match and its place by counting the smaller sites.
+    template<class W>
+    __device__ __forceinline__ uint32_t append_edges( W & w, NewEdges & ne, uint32_t j, uint32_t & err )
+    {
+        const uint32_t lane = lane_id();
+        uint32_t       written = 0;
+        if ( ne.count <= 32 )
+        {
+            const uint32_t v      = ne.slot[ 0 ];
+            const bool     has    = lane < ne.count;
+            const uint32_t key    = has ? v >> 2 : 0x80000000u | lane;
+            const uint32_t peers  = __match_any_sync( kFull, key );
+            const uint32_t two    = __ballot_sync( kFull, has && ( v & 2u ) );
+            const uint32_t closed = __ballot_sync( kFull, has && ( v & 1u ) );
+            const bool     first  = has && lane == __ffs( peers ) - 1;
+            uint32_t       groups = __ballot_sync( kFull, first );
+            written               = __popc( groups );
+            uint32_t rank         = 0;
+            while ( groups )
+            {
+                rank += __shfl_sync( kFull, key, __ffs( groups ) - 1 ) < key;
+                groups &= groups - 1;
+            }
+            if ( first )
+            {
+                const uint32_t dst = w.en + rank;
+                if ( dst < kEdgeSlots )
+                    w.e[ dst ] = make_uint4( min( j, key ), max( j, key ),
+                                             ( peers & closed ) && !( peers & two ) ? kNone : __popc( peers ), 0u );
+                else
+                    err |= kErrEdgeCap;
+            }
+            return written;
+        }
+        sort64( ne.slot );
+        const uint32_t next0 = ne.slot[ 1 ];
+        const uint32_t next1 = __shfl_down_sync( kFull, ne.slot[ 0 ], 1 );
+        const bool     last0 = ( ( next0 >> 2 ) != ( ne.slot[ 0 ] >> 2 ) ) && ( ne.slot[ 0 ] & 3u ) != 3u;
+        const bool     last1 = ( lane == 31 || ( next1 >> 2 ) != ( ne.slot[ 1 ] >> 2 ) ) && ( ne.slot[ 1 ] & 3u ) != 3u;
+        // index of the previous group end (exclusive max-scan over elements)
+        int prev = last1 ? int( 2 * lane + 1 ) : ( last0 ? int( 2 * lane ) : -1 );
+#pragma unroll 1
+        for ( int o = 1; o < 32; o <<= 1 )
+        {
+            const int y = __shfl_up_sync( kFull, prev, o );
+            if ( int( lane ) >= o )
+                prev = max( prev, y );
+        }
+        int before = __shfl_up_sync( kFull, prev, 1 );
+        if ( lane == 0 )
+            before = -1;
+        uint32_t woff = warp_exclusive_scan( uint32_t( last0 ) + uint32_t( last1 ), written );
+#pragma unroll
+        for ( uint32_t s = 0; s < 2; s++ )
+        {
+            const int      f = int( 2 * lane + s );
+            const uint32_t v = ne.slot[ s ];
+            if ( s ? last1 : last0 )
+            {
+                const uint32_t other = v >> 2;
+                const uint32_t dst   = w.en + woff;
+                if ( dst < kEdgeSlots )
+                    w.e[ dst ] = make_uint4( min( j, other ), max( j, other ), ( v & 1u ) ? kNone : uint32_t( f - before ), 0u );
+                else
+                    err |= kErrEdgeCap;
+                woff++;
+                before = f;
+            }
+        }
+        return written;
+    }
+
     // Flags a store that went past the reference's capacity; records written beyond the
     // shared slots are dropped.
-    __device__ __forceinline__ void check_capacity( const WarpCell & w, uint32_t & err )
+    template<class W>
+    __device__ __forceinline__ void check_capacity( const W & w, uint32_t & err )
     {
         if ( w.vn > kMaxVertices )
             err |= kErrVertexCap;
@@ -221,8 +396,17 @@ namespace apo2
 
     // -----------------------------------------------------------------------------------
     // Cell update: clip the cell of site i by site j (topology_update.inl:49-555)
+    //
+    // Bound by instruction fetch before anything else: the 16 warps of an SM are each at another
+    // place of some two thousand instructions, most run once per update (7.0 of the 13.4 cycles
+    // between two issues of a warp were waits for instructions). So loops stay rolled, the FP32
+    // form is an instantiation of its own, and code that both roots, both sites of an edge or both
+    // solves need is there once. With the neighbour list this took the 1M-site protein packing's
+    // kNN cells from 129 to 71 ms and its vertex validation from 265 to 189 ms, the 1M log-normal
+    // cloud's from 115 to 61 and from 140 to 106 ms; waits for instructions are 1.7 of 9.2 cycles.
     // -----------------------------------------------------------------------------------
-    __device__ bool update_cell( const CellContext & c, WarpCell & w, uint32_t i, double4 si, uint32_t j, double4 sj,
+    template<bool Fp32>
+    __device__ bool update_cell( const CellContext & c, WarpCell<Fp32> & w, uint32_t i, double4 si, uint32_t j, double4 sj,
                                  uint32_t & err )
     {
         const uint32_t lane = lane_id();
@@ -239,6 +423,7 @@ namespace apo2
                     return false;
                 w.vn = 0;
                 w.en = 0;
+                w.un = 0;
                 return false;
             }
         }
@@ -249,25 +434,29 @@ namespace apo2
         ne.count     = 0;
 
         const uint32_t baseV = w.vn, baseE = w.en;
+        uint32_t       gone  = 0; // some vertex was marked, or some closed edge emptied
 
         // 1. Vertices inside sj are marked; each one removes a vertex from its three edges
         //    (:96-154). The 8-bit edge index of the reference is kept.
+#pragma unroll 1
         for ( uint32_t vs = 0; vs <= baseV / 32; vs++ )
         {
             const uint32_t id      = lane + 32 * vs;
             bool           invalid = false;
             if ( id < baseV )
             {
-                invalid = sphere_conflict( c, sj, w.pos[ id ], w.tally );
+                invalid = sphere_conflict<Fp32>( sj, w.pos[ id ], w.tally );
                 if ( invalid )
                     w.v[ id ].w |= 0xff00u;
             }
             uint32_t m = __ballot_sync( kFull, invalid );
+            gone |= m;
             while ( m )
             {
                 const uint32_t t = highest( m );
                 m &= ~( 1u << t );
                 const uint4 vx = w.v[ 32 * vs + t ];
+#pragma unroll 1
                 for ( uint32_t es = 0; es <= baseE / 32; es++ )
                 {
                     const uint8_t eid = uint8_t( lane + 32 * es );
@@ -285,6 +474,7 @@ namespace apo2
 
         // 2. New vertices on every edge (:156-323).
         uint32_t closed_bits = 0;
+#pragma unroll 1
         for ( uint32_t es = 0; es <= baseE / 32; es++ )
         {
             const uint32_t e   = lane + 32 * es;
@@ -302,48 +492,18 @@ namespace apo2
                 has  = mask != 0;
             }
             // a closed edge is emptied when its trisector point falls inside sj (:184-191)
+            bool emptied = false;
             if ( e < baseE && mask == 0 && r.z == kNone )
             {
                 trisector( si, sk, sl, q0, q0 );
-                if ( intersects( q0, sj ) )
+                emptied = intersects( q0, sj );
+                if ( emptied )
                     w.e[ e ].z = 0;
             }
+            gone |= __ballot_sync( kFull, emptied );
 
-            // The emptiness predicate of every root (topology_update.inl:577-590): on a small
-            // cell each lane checks its own roots against every edge site; on a large one the
-            // whole warp checks one root at a time, 32 edges per step.
-            uint32_t valid = mask;
-            if ( baseE <= kLaneClearEdges )
-            {
-                if ( has )
-                {
-                    if ( ( mask & 1u ) && !clear_by_lane( c, w, q0, k, l ) )
-                        valid &= ~1u;
-                    if ( ( mask & 2u ) && !clear_by_lane( c, w, q1, k, l ) )
-                        valid &= ~2u;
-                }
-            }
-            else
-            {
-                uint32_t hm = __ballot_sync( kFull, has );
-                while ( hm )
-                {
-                    const uint32_t t = highest( hm );
-                    hm &= ~( 1u << t );
-                    uint32_t       tm = __shfl_sync( kFull, mask, t );
-                    const uint32_t tk = __shfl_sync( kFull, k, t ), tl = __shfl_sync( kFull, l, t );
-                    while ( tm )
-                    {
-                        const uint32_t nv = __ffs( tm ) - 1;
-                        tm &= ~( 1u << nv );
-                        const double4 cand = shfl4( nv ? q1 : q0, t );
-                        const bool    ok   = edges_clear( c, w, cand, tk, tl );
-                        if ( lane == t && !ok )
-                            valid &= ~( 1u << nv );
-                    }
-                }
-            }
-
+            // the emptiness predicate of every root (topology_update.inl:577-590)
+            const uint32_t valid = spheres_clear( c, w, q0, q1, mask, k, l );
             const uint32_t count = __popc( valid );
             has                  = has && count > 0;
             if ( has )
@@ -353,61 +513,71 @@ namespace apo2
                     vnb = 0;
                 w.e[ e ].z = vnb + count;
             }
-            uint32_t total;
-            uint32_t off = warp_exclusive_scan( count, total );
+            // vertices of the lanes below, and of all lanes
+            const uint32_t one   = __ballot_sync( kFull, count >= 1 ), two = __ballot_sync( kFull, count == 2 );
+            const uint32_t below = ( 1u << lane ) - 1u;
+            const uint32_t total = __popc( one ) + __popc( two );
 
             // new vertex records with sorted ids, and their positions (:256-275)
-            uint32_t jj = j, kk = k, ll = l, t;
-            if ( jj > ll )
+            if ( has )
             {
-                t  = jj;
-                jj = ll;
-                ll = t;
-            }
-            if ( jj > kk )
-            {
-                t  = jj;
-                jj = kk;
-                kk = t;
-            }
-            if ( kk > ll )
-            {
-                t  = kk;
-                kk = ll;
-                ll = t;
-            }
-            uint32_t vm = valid;
-            while ( vm )
-            {
-                const uint32_t nv = __ffs( vm ) - 1;
-                vm &= ~( 1u << nv );
-                const uint32_t dst = w.vn + off;
-                if ( dst < kVertexSlots )
+                uint32_t jj = j, kk = k, ll = l, t;
+                if ( jj > ll )
                 {
-                    w.v[ dst ] = make_uint4( jj, kk, ll, nv );
-                    // same call as a later re-solve when the new site is the smallest id
-                    w.pos[ dst ] = ( jj == j ) ? ( nv ? q1 : q0 ) : solve_vertex( c, si, make_uint4( jj, kk, ll, nv ) );
+                    t  = jj;
+                    jj = ll;
+                    ll = t;
                 }
-                else
-                    err |= kErrVertexCap;
-                off++;
+                if ( jj > kk )
+                {
+                    t  = jj;
+                    jj = kk;
+                    kk = t;
+                }
+                if ( kk > ll )
+                {
+                    t  = kk;
+                    kk = ll;
+                    ll = t;
+                }
+                // same call as a later re-solve when the new site is the smallest id
+                if ( jj != j )
+                {
+                    q0 = q1 = make_double4( 0, 0, 0, 0 );
+                    quadrisector( si, site( c, jj ), site( c, kk ), site( c, ll ), q0, q1 );
+                }
+                uint32_t dst = w.vn + __popc( one & below ) + __popc( two & below );
+#pragma unroll 1
+                for ( uint32_t nv = 0; nv < 2; nv++ )
+                {
+                    if ( !( ( valid >> nv ) & 1u ) )
+                        continue;
+                    if ( dst < kVertexSlots )
+                    {
+                        w.v[ dst ]   = make_uint4( jj, kk, ll, nv );
+                        w.pos[ dst ] = nv ? q1 : q0;
+                    }
+                    else
+                        err |= kErrVertexCap;
+                    dst++;
+                }
             }
 
-            // two new-edge candidates per new vertex, lanes from the highest (:277-316)
-            uint32_t lm = __ballot_sync( kFull, valid != 0 );
+            // two new-edge candidates per new vertex (:277-316)
+            const uint32_t pk = pack_edge( k, count == 2, false ), pl = pack_edge( l, count == 2, false );
+            uint32_t       lm = one;
             while ( lm )
             {
-                const uint32_t tl2 = highest( lm );
-                lm &= ~( 1u << tl2 );
-                uint32_t       tv = __shfl_sync( kFull, valid, tl2 );
-                const uint32_t tc = __shfl_sync( kFull, count, tl2 );
-                const uint32_t tk = __shfl_sync( kFull, k, tl2 ), tl = __shfl_sync( kFull, l, tl2 );
-                while ( tv )
+                const uint32_t t = highest( lm );
+                const uint32_t a = __shfl_sync( kFull, pk, t ), b = __shfl_sync( kFull, pl, t );
+                ne.push( a, err );
+                ne.push( b, err );
+                if ( a & 2u )
                 {
-                    tv &= tv - 1;
-                    ne.push( tk, tc == 2, false, err );
-                    ne.push( tl, tc == 2, false, err );
+                    ne.push( a, err );
+                    ne.push( b, err );
                 }
+                lm &= ~( 1u << t );
             }
             w.vn += total;
             closed_bits = ( closed_bits | ( ( e < baseE && mask == 0 ) ? ( 1u << es ) : 0u ) ) & 0xffu;
@@ -418,6 +588,7 @@ namespace apo2
         // 3. Closed elliptic trisectors with the sites of edges that got no vertex (:325-433).
         if ( __any_sync( kFull, closed_bits != 0 ) )
         {
+#pragma unroll 1
             for ( uint32_t es = 0; es <= baseE / 32; es++ )
             {
                 const bool can = ( closed_bits >> es ) & 1u;
@@ -425,93 +596,49 @@ namespace apo2
                     continue;
                 const uint32_t e = lane + 32 * es;
                 const uint4    r = e < kEdgeSlots ? w.e[ e ] : make_uint4( 0, 0, 0, 0 );
-                double4        sites2[ 2 ] = { make_double4( 0, 0, 0, 0 ), make_double4( 0, 0, 0, 0 ) };
-                if ( e < baseE )
-                {
-                    sites2[ 0 ] = site( c, r.x );
-                    sites2[ 1 ] = site( c, r.y );
-                }
+#pragma unroll 1
                 for ( uint32_t s = 0; s < 2; s++ )
                 {
                     const uint32_t id  = s ? r.y : r.x;
                     bool           cur = can;
-                    uint32_t       cm  = __ballot_sync( kFull, cur );
-                    while ( cm )
+                    // a site that is a candidate already (with a vertex or as a closed edge) is out
+#pragma unroll 1
+                    for ( uint32_t q = 0; q < min( ne.count, kMaxNewEdges ); q++ )
                     {
-                        const uint32_t t = highest( cm );
-                        cm &= ~( 1u << t );
-                        const uint32_t tid = __shfl_sync( kFull, id, t );
-                        const bool     shared = ne.contains( tid );
-                        if ( lane == t && shared )
-                            cur = false;
+                        const uint32_t taken = __shfl_sync( kFull, q < 32 ? ne.slot[ 0 ] : ne.slot[ 1 ], q & 31u ) >> 2;
+                        cur                  = cur && taken != id;
                     }
                     double4  x0 = make_double4( 0, 0, 0, 0 ), x1 = make_double4( 0, 0, 0, 0 );
                     uint32_t cnt = 0;
                     if ( cur )
-                        cnt = trisector( si, sj, sites2[ s ], x0, x1 );
-                    cur = cur && cnt == 2;
-                    cm  = __ballot_sync( kFull, cur );
+                        cnt = trisector( si, sj, site( c, id ), x0, x1 );
+                    uint32_t cm = __ballot_sync( kFull, cur && cnt == 2 );
                     while ( cm )
                     {
-                        const uint32_t t = highest( cm );
+                        const uint32_t t   = highest( cm );
                         cm &= ~( 1u << t );
                         const uint32_t tid = __shfl_sync( kFull, id, t );
-                        const double4  tv  = shfl4( x0, t );
-                        if ( edges_clear( c, w, tv, tid, i ) )
-                            ne.push( tid, false, true, err );
+                        if ( edges_clear( c, w, shfl4( x0, t ), tid, i ) )
+                            ne.push( pack_edge( tid, false, true ), err );
                     }
                 }
             }
         }
 
         // 4. Unique new edges by site, with the number of new vertices on each (:435-515).
-        sort64( ne.slot );
-        const uint32_t next0 = ne.slot[ 1 ];
-        const uint32_t next1 = __shfl_down_sync( kFull, ne.slot[ 0 ], 1 );
-        const bool     last0 = ( ( next0 >> 2 ) != ( ne.slot[ 0 ] >> 2 ) ) && ( ne.slot[ 0 ] & 3u ) != 3u;
-        const bool     last1 = ( lane == 31 || ( next1 >> 2 ) != ( ne.slot[ 1 ] >> 2 ) ) && ( ne.slot[ 1 ] & 3u ) != 3u;
-        // index of the previous group end (exclusive max-scan over elements)
-        int lane_last = last1 ? int( 2 * lane + 1 ) : ( last0 ? int( 2 * lane ) : -1 );
-        int prev      = lane_last;
-#pragma unroll
-        for ( int o = 1; o < 32; o <<= 1 )
-        {
-            const int y = __shfl_up_sync( kFull, prev, o );
-            if ( int( lane ) >= o )
-                prev = max( prev, y );
-        }
-        int before = __shfl_up_sync( kFull, prev, 1 );
-        if ( lane == 0 )
-            before = -1;
-        uint32_t written;
-        uint32_t woff = warp_exclusive_scan( uint32_t( last0 ) + uint32_t( last1 ), written );
-        for ( uint32_t s = 0; s < 2; s++ )
-        {
-            const bool     isLast = s ? last1 : last0;
-            const int      f      = int( 2 * lane + s );
-            const uint32_t v      = ne.slot[ s ];
-            if ( isLast )
-            {
-                const uint32_t other = v >> 2;
-                const uint32_t dst   = w.en + woff;
-                if ( dst < kEdgeSlots )
-                    w.e[ dst ] = make_uint4( min( j, other ), max( j, other ), ( v & 1u ) ? kNone : uint32_t( f - before ), 0u );
-                else
-                    err |= kErrEdgeCap;
-                woff++;
-                before = f;
-            }
-        }
+        const uint32_t written = append_edges( w, ne, j, err );
         w.en += written;
         check_capacity( w, err );
         w.vn = min( w.vn, kVertexSlots );
         w.en = min( w.en, kEdgeSlots );
         __syncwarp();
 
-        // 5. Stable compaction of the marked vertices and the emptied edges (:520-542).
-        if ( w.vn > 0 )
+        // 5. Stable compaction of the marked vertices and the emptied edges (:520-542); without
+        //    any, every record stays where it is.
+        if ( gone )
         {
             uint32_t kept = 0;
+#pragma unroll 1
             for ( uint32_t base = 0; base < w.vn; base += 32 )
             {
                 const uint32_t id   = base + lane;
@@ -536,9 +663,8 @@ namespace apo2
                 __syncwarp();
             }
             w.vn = kept;
-        }
-        {
-            uint32_t kept = 0;
+            kept = 0;
+#pragma unroll 1
             for ( uint32_t base = 0; base < w.en; base += 32 )
             {
                 const uint32_t id   = base + lane;
@@ -559,11 +685,14 @@ namespace apo2
             }
             w.en = kept;
         }
+        if ( gone || written )
+            relist_sites( w, j );
         return written != 0;
     }
 
     // Largest vertex or closed-trisector radius of the cell (topology_update.inl:595-653).
-    __device__ double cell_radius( const CellContext & c, const WarpCell & w, double4 si )
+    template<class W>
+    __device__ double cell_radius( const CellContext & c, const W & w, double4 si )
     {
         double m = 0.0;
         for ( uint32_t base = 0; base < w.vn; base += 32 )
@@ -592,20 +721,24 @@ namespace apo2
     // -----------------------------------------------------------------------------------
     // Shared-memory carving and the per-cell store
     // -----------------------------------------------------------------------------------
-    __device__ __forceinline__ WarpCell carve( unsigned char * smem, uint32_t warp, uint32_t extra )
+    template<bool Fp32>
+    __device__ __forceinline__ WarpCell<Fp32> carve( unsigned char * smem, uint32_t warp, uint32_t extra )
     {
         unsigned char * base = smem + size_t( warp ) * ( kWarpCellBytes + extra );
-        WarpCell        w;
+        WarpCell<Fp32>  w;
         w.pos = reinterpret_cast<double4 *>( base );
         w.v   = reinterpret_cast<uint4 *>( base + sizeof( double4 ) * kVertexSlots );
         w.e   = reinterpret_cast<uint4 *>( base + ( sizeof( double4 ) + sizeof( uint4 ) ) * kVertexSlots );
+        w.u   = reinterpret_cast<uint32_t *>( w.e + kEdgeSlots );
         w.vn    = 0;
         w.en    = 0;
+        w.un    = 0;
         w.tally = FilterTally {};
         return w;
     }
 
-    __device__ __forceinline__ void load_cell( const CellContext & c, WarpCell & w, uint32_t i, double4 si, bool with_vertices,
+    template<class W>
+    __device__ __forceinline__ void load_cell( const CellContext & c, W & w, uint32_t i, double4 si, bool with_vertices,
                                                bool solve )
     {
         w.en = c.edge_nb[ i ];
@@ -624,9 +757,11 @@ namespace apo2
             }
         }
         __syncwarp();
+        list_sites( w );
     }
 
-    __device__ __forceinline__ void store_cell( const CellContext & c, const WarpCell & w, uint32_t i, uint32_t vertex_base,
+    template<class W>
+    __device__ __forceinline__ void store_cell( const CellContext & c, const W & w, uint32_t i, uint32_t vertex_base,
                                                 uint32_t & err )
     {
         const uint32_t vn = min( vertex_base + w.vn, kMaxVertices );
@@ -653,10 +788,11 @@ namespace apo2
             atomicOr( c.error, err );
     }
     // Error flags and the FP32 filter's counts of a warp at the end of a kernel.
-    __device__ __forceinline__ void report( const CellContext & c, uint32_t err, const WarpCell & w )
+    template<bool Fp32>
+    __device__ __forceinline__ void report( const CellContext & c, uint32_t err, const WarpCell<Fp32> & w )
     {
         report( c, err );
-        if ( c.fp32 && c.counters )
+        if ( Fp32 && c.counters )
         {
             const uint32_t tests = __reduce_add_sync( kFull, w.tally.tests );
             const uint32_t esc   = __reduce_add_sync( kFull, w.tally.escalated );
@@ -860,7 +996,8 @@ namespace apo2
     __constant__ uint32_t c_initial_edges[ 12 ][ 2 ] = { { 0, 2 }, { 2, 4 }, { 1, 2 }, { 2, 5 }, { 1, 4 }, { 1, 5 },
                                                          { 0, 5 }, { 0, 4 }, { 1, 3 }, { 3, 5 }, { 0, 3 }, { 3, 4 } };
 
-    __device__ __forceinline__ void initial_cell( const CellContext & c, WarpCell & w, double4 si )
+    template<class W>
+    __device__ __forceinline__ void initial_cell( const CellContext & c, W & w, double4 si )
     {
         // 8 vertices and 12 edges on the artificial sites (algorithm.inl:1466-1505)
         const uint32_t n    = c.n;
@@ -873,8 +1010,11 @@ namespace apo2
         }
         if ( lane < 12 )
             w.e[ lane ] = make_uint4( n + c_initial_edges[ lane ][ 0 ], n + c_initial_edges[ lane ][ 1 ], 2u, 0u );
+        if ( lane < kArtificial )
+            w.u[ lane ] = n + lane;
         w.vn = 8;
         w.en = 12;
+        w.un = kArtificial;
         __syncwarp();
     }
 
@@ -883,13 +1023,14 @@ namespace apo2
     // initializeDataStructure, topology_update.inl:5-47, fused in); kCellsNext continues the
     // stored cells with the next kNN step; kCellsInitOnly writes the initial cells, statuses
     // and known radii alone (no kNN step at all).
+    template<bool Fp32>
     __global__ void __launch_bounds__( kCellBlock, 4 ) k_cells( CellContext c, uint32_t mode )
     {
         extern __shared__ __align__( 16 ) unsigned char smem[];
         const uint32_t warp  = threadIdx.x >> 5;
         const uint32_t gwarp = blockIdx.x * ( kCellBlock / 32 ) + warp;
         const uint32_t nwarp = gridDim.x * ( kCellBlock / 32 );
-        WarpCell       w     = carve( smem, warp, 0 );
+        WarpCell<Fp32> w = carve<Fp32>( smem, warp, 0 );
         uint32_t       err   = 0;
         // per-warp counters (lane 0 counts), added to the build's counters at the end
         __shared__ uint32_t s_counts[ kCellBlock / 32 ][ kCounters ];
@@ -1009,13 +1150,14 @@ namespace apo2
     // whether that neighbour changed the cell and whether the security-radius certificate held
     // after it. A cell stops at the rank where it certifies (and is then FullyValidated). Row i
     // of `contributed` / `certified` holds steps x k bytes; this step writes its k.
+    template<bool Fp32>
     __global__ void __launch_bounds__( kCellBlock, 4 ) k_cells_profile( CellContext c, uint32_t step, uint32_t row,
                                                                        uint8_t * __restrict__ contributed,
                                                                        uint8_t * __restrict__ certified )
     {
         extern __shared__ __align__( 16 ) unsigned char smem[];
         const uint32_t warp = threadIdx.x >> 5;
-        WarpCell       w    = carve( smem, warp, 0 );
+        WarpCell<Fp32> w = carve<Fp32>( smem, warp, 0 );
         uint32_t       err  = 0;
         while ( true )
         {
@@ -1074,6 +1216,7 @@ namespace apo2
     // -----------------------------------------------------------------------------------
     // Vertex validation (algorithm.inl:208-476)
     // -----------------------------------------------------------------------------------
+    template<bool Fp32>
     __global__ void __launch_bounds__( kCellBlock, 4 ) k_vertex_validation( CellContext c, const uint32_t * __restrict__ tasks,
                                                                         const uint32_t * __restrict__ task_count )
     {
@@ -1082,7 +1225,7 @@ namespace apo2
         const uint32_t gwarp = blockIdx.x * ( kCellBlock / 32 ) + warp;
         const uint32_t nwarp = gridDim.x * ( kCellBlock / 32 );
         const uint32_t lane  = lane_id();
-        WarpCell       w     = carve( smem, warp, 0 );
+        WarpCell<Fp32> w = carve<Fp32>( smem, warp, 0 );
         uint32_t       err   = 0;
         const uint32_t count = *task_count;
         const uint32_t n     = c.n;
@@ -1303,7 +1446,8 @@ namespace apo2
     // node, then its stack from the top), `count` entries, earliest first.
     // One frontier node of the ordered walk: an internal node gives its entered children in walk
     // order (kids, first, second), a leaf whether it contributes.
-    __device__ __forceinline__ void ordered_step( const CellContext & c, const WarpCell & w, uint32_t i, double4 si,
+    template<class W>
+    __device__ __forceinline__ void ordered_step( const CellContext & c, const W & w, uint32_t i, double4 si,
                                                   const EdgeWalk & p, uint32_t node, uint32_t & kids, uint32_t & first,
                                                   uint32_t & second, bool & contrib, uint32_t & j )
     {
@@ -1382,7 +1526,8 @@ namespace apo2
     // is it or a leaf under one of the q nodes before it: everything after it is dropped and
     // the walk continues over those. `saved` holds the suspended lane's position (its current
     // node, then its stack from the top), `count` entries, earliest first.
-    __device__ uint32_t ordered_edge_walk( const CellContext & c, const WarpCell & w, uint32_t i, double4 si, const EdgeWalk & p,
+    template<class W>
+    __device__ uint32_t ordered_edge_walk( const CellContext & c, const W & w, uint32_t i, double4 si, const EdgeWalk & p,
                                            uint32_t * frontier, const uint32_t * saved, uint32_t count, uint32_t & err )
     {
         const uint32_t lane = lane_id();
@@ -1458,6 +1603,7 @@ namespace apo2
         return found;
     }
 
+    template<bool Fp32>
     __global__ void __launch_bounds__( kCellBlock, 4 ) k_edge_validation( CellContext c, const uint32_t * __restrict__ tasks,
                                                                       const uint32_t * __restrict__ task_count,
                                                                       SearchProof proof )
@@ -1467,7 +1613,7 @@ namespace apo2
         const uint32_t gwarp = blockIdx.x * ( kCellBlock / 32 ) + warp;
         const uint32_t nwarp = gridDim.x * ( kCellBlock / 32 );
         const uint32_t lane  = lane_id();
-        WarpCell       w     = carve( smem, warp, 0 );
+        WarpCell<Fp32> w = carve<Fp32>( smem, warp, 0 );
         uint32_t       err   = 0;
         const uint32_t count = *task_count;
         const uint32_t n     = c.n;
@@ -1724,8 +1870,8 @@ namespace apo2
                             tm &= ~( 1u << nv );
                             const double4  cand = shfl4( nv ? x1 : x0, t2 );
                             const uint32_t h0 = __shfl_sync( kFull, hint0, t2 ), h1 = __shfl_sync( kFull, hint1, t2 );
-                            const bool     hinted = pristine && ( ( h0 != kNone && site_conflict( c, h0, cand, w.tally ) )
-                                                              || ( h1 != kNone && site_conflict( c, h1, cand, w.tally ) ) );
+                            const bool     hinted = pristine && ( ( h0 != kNone && site_conflict<Fp32>( c, h0, cand, w.tally ) )
+                                                              || ( h1 != kNone && site_conflict<Fp32>( c, h1, cand, w.tally ) ) );
                             const bool     ok   = !hinted && edges_clear( c, w, cand, tk, tl );
                             if ( lane == t2 && !ok )
                                 valid &= ~( 1u << nv );
@@ -1818,13 +1964,14 @@ namespace apo2
     // -----------------------------------------------------------------------------------
     // Cells are taken one at a time from a shared counter: their costs are uneven (a few hold
     // long searches), and a fixed share per warp left most warps idle at the end.
+    template<bool Fp32>
     __global__ void __launch_bounds__( kCellBlock, 3 ) k_bisector_validation( CellContext c, uint32_t * __restrict__ next )
     {
         extern __shared__ __align__( 16 ) unsigned char smem[];
         const uint32_t warp  = threadIdx.x >> 5;
         const uint32_t lane  = lane_id();
-        WarpCell       w     = carve( smem, warp, kBisectorBytes );
-        uint32_t *     bis   = reinterpret_cast<uint32_t *>( reinterpret_cast<unsigned char *>( w.e ) + sizeof( uint4 ) * kEdgeSlots );
+        WarpCell<Fp32> w = carve<Fp32>( smem, warp, kBisectorBytes );
+        uint32_t *     bis   = reinterpret_cast<uint32_t *>( reinterpret_cast<unsigned char *>( w.u ) + sizeof( uint32_t ) * kSiteSlots );
         uint32_t       err   = 0;
         const uint32_t n     = c.n;
         while ( true )
@@ -2330,13 +2477,21 @@ namespace apo2
             const int dev = current_device();
             int       sms = 148;
             cudaDeviceGetAttribute( &sms, cudaDevAttrMultiProcessorCount, dev );
-            cudaFuncSetAttribute( k_cells, cudaFuncAttributeMaxDynamicSharedMemorySize, int( cell_smem_bytes( false ) ) );
-            cudaFuncSetAttribute( k_cells_profile, cudaFuncAttributeMaxDynamicSharedMemorySize, int( cell_smem_bytes( false ) ) );
-            cudaFuncSetAttribute( k_vertex_validation, cudaFuncAttributeMaxDynamicSharedMemorySize, int( cell_smem_bytes( false ) ) );
-            cudaFuncSetAttribute( k_edge_validation, cudaFuncAttributeMaxDynamicSharedMemorySize, int( cell_smem_bytes( false ) ) );
-            cudaFuncSetAttribute( k_bisector_validation, cudaFuncAttributeMaxDynamicSharedMemorySize, int( cell_smem_bytes( true ) ) );
+            const auto room = []( auto * kernel, bool bisector ) {
+                cudaFuncSetAttribute( kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int( cell_smem_bytes( bisector ) ) );
+            };
+            room( k_cells<false>, false );
+            room( k_cells<true>, false );
+            room( k_cells_profile<false>, false );
+            room( k_cells_profile<true>, false );
+            room( k_vertex_validation<false>, false );
+            room( k_vertex_validation<true>, false );
+            room( k_edge_validation<false>, false );
+            room( k_edge_validation<true>, false );
+            room( k_bisector_validation<false>, true );
+            room( k_bisector_validation<true>, true );
             int per_sm = 0;
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor( &per_sm, k_cells, kCellBlock, cell_smem_bytes( false ) );
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor( &per_sm, k_cells<false>, kCellBlock, cell_smem_bytes( false ) );
             cell_grid_slot() = sms * std::max( 1, per_sm );
         } );
         if ( cell_grid_slot() == 0 ) // an ordinal outside the table: size it for 148 SMs x 4 blocks
@@ -2368,7 +2523,7 @@ namespace apo2
     void launch_cells( const CellContext & c, uint32_t mode, cudaStream_t s )
     {
         cudaMemsetAsync( c.work_counter, 0, sizeof( uint32_t ), s );
-        APO2_LAUNCH( "k_cells", s, k_cells<<<cell_grid( c.n ), kCellBlock, cell_smem_bytes( false ), s>>>( c, mode ) );
+        APO2_LAUNCH( "k_cells", s, ( c.fp32 ? k_cells<true> : k_cells<false> )<<<cell_grid( c.n ), kCellBlock, cell_smem_bytes( false ), s>>>( c, mode ) );
     }
 
     void launch_cells_profile( const CellContext & c, uint32_t step, uint32_t row, uint8_t * contributed, uint8_t * certified,
@@ -2377,7 +2532,7 @@ namespace apo2
         configure_cell_kernels();
         cudaMemsetAsync( c.work_counter, 0, sizeof( uint32_t ), s );
         APO2_LAUNCH( "k_cells_profile", s,
-                     k_cells_profile<<<cell_grid( c.n ), kCellBlock, cell_smem_bytes( false ), s>>>( c, step, row, contributed, certified ) );
+                     ( c.fp32 ? k_cells_profile<true> : k_cells_profile<false> )<<<cell_grid( c.n ), kCellBlock, cell_smem_bytes( false ), s>>>( c, step, row, contributed, certified ) );
     }
 
     void launch_tasks( const CellContext & c, uint32_t * tasks, uint32_t * count, cudaStream_t s )
@@ -2389,20 +2544,20 @@ namespace apo2
     void launch_vertex_validation( const CellContext & c, const uint32_t * tasks, const uint32_t * count, cudaStream_t s )
     {
         cudaMemsetAsync( c.work_counter, 0, sizeof( uint32_t ), s );
-        APO2_LAUNCH( "k_vertex_validation", s, k_vertex_validation<<<cell_grid( c.n ), kCellBlock, cell_smem_bytes( false ), s>>>( c, tasks, count ) );
+        APO2_LAUNCH( "k_vertex_validation", s, ( c.fp32 ? k_vertex_validation<true> : k_vertex_validation<false> )<<<cell_grid( c.n ), kCellBlock, cell_smem_bytes( false ), s>>>( c, tasks, count ) );
     }
 
     void launch_edge_validation( const CellContext & c, const uint32_t * tasks, const uint32_t * count, cudaStream_t s,
                                  SearchProof proof )
     {
         cudaMemsetAsync( c.work_counter, 0, sizeof( uint32_t ), s );
-        APO2_LAUNCH( "k_edge_validation", s, k_edge_validation<<<cell_grid( c.n ), kCellBlock, cell_smem_bytes( false ), s>>>( c, tasks, count, proof ) );
+        APO2_LAUNCH( "k_edge_validation", s, ( c.fp32 ? k_edge_validation<true> : k_edge_validation<false> )<<<cell_grid( c.n ), kCellBlock, cell_smem_bytes( false ), s>>>( c, tasks, count, proof ) );
     }
 
     void launch_bisector_validation( const CellContext & c, cudaStream_t s )
     {
         cudaMemsetAsync( c.work_counter, 0, sizeof( uint32_t ), s );
-        APO2_LAUNCH( "k_bisector_validation", s, k_bisector_validation<<<cell_grid( c.n ), kCellBlock, cell_smem_bytes( true ), s>>>( c, c.work_counter ) );
+        APO2_LAUNCH( "k_bisector_validation", s, ( c.fp32 ? k_bisector_validation<true> : k_bisector_validation<false> )<<<cell_grid( c.n ), kCellBlock, cell_smem_bytes( true ), s>>>( c, c.work_counter ) );
     }
 
     void launch_output( const CellContext & c, const OutputBuffers & o, cudaStream_t s )

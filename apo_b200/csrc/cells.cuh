@@ -15,7 +15,12 @@ namespace apo2
     // update appends before it compacts; writes past the slots are dropped and flagged.
     constexpr uint32_t kVertexSlots   = 192;
     constexpr uint32_t kEdgeSlots     = 296;
-    constexpr size_t   kWarpCellBytes = ( sizeof( double4 ) + sizeof( uint4 ) ) * kVertexSlots + sizeof( uint4 ) * kEdgeSlots;
+    // Slots of the cell's neighbour list: what the 57,344 bytes a block may have at four blocks per
+    // SM leave over. A cell of simple vertices with E edges has E / 3 + 2 neighbours, so only cells
+    // above 230 edges (of 264) can outgrow it; their edges are scanned instead.
+    constexpr uint32_t kSiteSlots     = 80;
+    constexpr size_t   kWarpCellBytes = ( sizeof( double4 ) + sizeof( uint4 ) ) * kVertexSlots + sizeof( uint4 ) * kEdgeSlots
+                                      + sizeof( uint32_t ) * kSiteSlots;
     constexpr size_t   kBisectorBytes = sizeof( uint32_t ) * 2 * kMaxBisectors;
     static_assert( kWarpCellBytes % 32 == 0, "warp cell must keep double4 alignment" );
 
@@ -72,10 +77,12 @@ namespace apo2
     };
 
     // The reference's conflict test of site `id` against the sphere x (gpu/math.cuh:374-388),
-    // decided by the FP32 filter where it can in the filtered form.
+    // decided by the FP32 filter where it can in the filtered form (Fp32: a kernel instantiation of
+    // its own, so that neither form carries the other's code through the instruction cache).
+    template<bool Fp32>
     __device__ __forceinline__ bool site_conflict( const CellContext & c, uint32_t id, double4 x, FilterTally & t )
     {
-        if ( c.fp32 )
+        if constexpr ( Fp32 )
         {
             t.tests++;
             // the float copy holds the n input sites; the six bounding sites are rounded here
@@ -85,12 +92,13 @@ namespace apo2
                 return f == 1;
             t.escalated++;
         }
-        return intersects( c.sites[ id ], x );
+        return intersects_wide( c.sites[ id ], x );
     }
     // The same for a site given by value (its float copy is exact for float input and bounded otherwise).
-    __device__ __forceinline__ bool sphere_conflict( const CellContext & c, double4 site, double4 x, FilterTally & t )
+    template<bool Fp32>
+    __device__ __forceinline__ bool sphere_conflict( double4 site, double4 x, FilterTally & t )
     {
-        if ( c.fp32 )
+        if constexpr ( Fp32 )
         {
             t.tests++;
             const int f = conflict_filter( to_float( site ), x );
@@ -98,7 +106,7 @@ namespace apo2
                 return f == 1;
             t.escalated++;
         }
-        return intersects( site, x );
+        return intersects_wide( site, x );
     }
 
     // Row of cell i in the per-cell stores (vertices, edges), which hold only the cells

@@ -108,6 +108,29 @@ namespace apo2
     }
     __device__ __forceinline__ bool intersects( double4 a, double4 b ) { return lt_eps( sphere_distance( a, b ), 0. ); }
 
+    // intersects( a, b ) without the conversions and the single-precision root wherever the
+    // squared distance alone decides it. The reference's distance is the root of |a - b|^2 rounded
+    // to float, taken with the approximate unit: within 4e-7 of the exact one, so a squared distance
+    // more than 1e-5 (relative) away from (ra + rb)^2 is on the same side of the 1e-8 comparison
+    // once ra + rb is above 1e-2. Anything nearer, a smaller or negative sum, a squared distance
+    // that float may not hold, and NaN take the reference's own arithmetic. A float conversion or
+    // a root takes four times the issue slots of an FP64 operation, and the predicate needs three.
+    __device__ __forceinline__ bool intersects_wide( double4 a, double4 b )
+    {
+        const double dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z;
+        const double dd = dx * dx + dy * dy + dz * dz;
+        const double s  = a.w + b.w;
+        const double t  = s * s;
+        if ( s > 1e-2 && dd < 1e37 )
+        {
+            if ( dd > t * 1.00001 )
+                return false;
+            if ( dd < t * 0.99999 )
+                return true;
+        }
+        return intersects( a, b );
+    }
+
     // FP32 static filter of the conflict predicate intersects(site, x) above, as the reference
     // evaluates it: d = double(sqrtf(float(|c - x|^2))) - (r + w) < 1e-8, with the approximate
     // single-precision square root of --use_fast_math. The filter recomputes d from the float

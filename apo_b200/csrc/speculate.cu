@@ -299,12 +299,14 @@ namespace apo2
             bool ok = true;
             for ( uint32_t h = 0; h < 2 && ok; h++ )
                 if ( hint_ok[ h ] )
-                    ok = !site_conflict( c, s.hint[ h ], x[ r ], untallied );
+                    ok = !( c.fp32 ? site_conflict<true>( c, s.hint[ h ], x[ r ], untallied )
+                                   : site_conflict<false>( c, s.hint[ h ], x[ r ], untallied ) );
             for ( uint32_t q = 0; q < s.nbr_count && ok; q++ )
             {
                 const uint32_t u = s.nbr[ q ];
                 if ( u != s.k && u != s.l )
-                    ok = !site_conflict( c, u, x[ r ], untallied );
+                    ok = !( c.fp32 ? site_conflict<true>( c, u, x[ r ], untallied )
+                                   : site_conflict<false>( c, u, x[ r ], untallied ) );
             }
             if ( ok )
                 return true;
