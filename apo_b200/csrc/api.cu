@@ -272,8 +272,10 @@ namespace
         if ( stop == 0 )
             launch_tasks( h->cells, h->tasks, h->task_counts + rounds, s );
         record( h, 5, s );
-        if ( stop == 0 )
-            launch_bisector_validation( h->cells, s );
+        if ( stop == 0 && h->options.edge_search == 1 )
+            launch_bisector_validation( h->cells, nullptr, nullptr, s );
+        else if ( stop == 0 )
+            launch_bisector_validation_speculative( h->cells, h->spec, s );
         record( h, 6, s );
         const cudaError_t err = cudaGetLastError();
         if ( err != cudaSuccess )

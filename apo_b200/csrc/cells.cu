@@ -1965,7 +1965,8 @@ namespace apo2
     // Cells are taken one at a time from a shared counter: their costs are uneven (a few hold
     // long searches), and a fixed share per warp left most warps idle at the end.
     template<bool Fp32>
-    __global__ void __launch_bounds__( kCellBlock, 3 ) k_bisector_validation( CellContext c, uint32_t * __restrict__ next )
+    __global__ void __launch_bounds__( kCellBlock, 3 ) k_bisector_validation( CellContext c, const uint32_t * __restrict__ tasks,
+                                                                          const uint32_t * __restrict__ task_count )
     {
         extern __shared__ __align__( 16 ) unsigned char smem[];
         const uint32_t warp  = threadIdx.x >> 5;
@@ -1974,14 +1975,16 @@ namespace apo2
         uint32_t *     bis   = reinterpret_cast<uint32_t *>( reinterpret_cast<unsigned char *>( w.u ) + sizeof( uint32_t ) * kSiteSlots );
         uint32_t       err   = 0;
         const uint32_t n     = c.n;
+        const uint32_t count = tasks ? *task_count : c.hi - c.lo;
         while ( true )
         {
-            uint32_t i = 0;
+            uint32_t t = 0;
             if ( lane == 0 )
-                i = c.lo + atomicAdd( next, 1u );
-            i = __shfl_sync( kFull, i, 0 );
-            if ( i >= c.hi )
+                t = atomicAdd( c.work_counter, 1u );
+            t = __shfl_sync( kFull, t, 0 );
+            if ( t >= count )
                 break;
+            const uint32_t i = tasks ? tasks[ t ] : c.lo + t;
             if ( c.status[ i ] == kBuried )
                 continue;
             const float   known = c.known_radii[ i ];
@@ -2554,10 +2557,10 @@ namespace apo2
         APO2_LAUNCH( "k_edge_validation", s, ( c.fp32 ? k_edge_validation<true> : k_edge_validation<false> )<<<cell_grid( c.n ), kCellBlock, cell_smem_bytes( false ), s>>>( c, tasks, count, proof ) );
     }
 
-    void launch_bisector_validation( const CellContext & c, cudaStream_t s )
+    void launch_bisector_validation( const CellContext & c, const uint32_t * tasks, const uint32_t * count, cudaStream_t s )
     {
         cudaMemsetAsync( c.work_counter, 0, sizeof( uint32_t ), s );
-        APO2_LAUNCH( "k_bisector_validation", s, ( c.fp32 ? k_bisector_validation<true> : k_bisector_validation<false> )<<<cell_grid( c.n ), kCellBlock, cell_smem_bytes( true ), s>>>( c, c.work_counter ) );
+        APO2_LAUNCH( "k_bisector_validation", s, ( c.fp32 ? k_bisector_validation<true> : k_bisector_validation<false> )<<<cell_grid( c.n ), kCellBlock, cell_smem_bytes( true ), s>>>( c, tasks, count ) );
     }
 
     void launch_output( const CellContext & c, const OutputBuffers & o, cudaStream_t s )

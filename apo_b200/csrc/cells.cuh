@@ -197,7 +197,8 @@ namespace apo2
     };
     void launch_edge_validation( const CellContext & c, const uint32_t * tasks, const uint32_t * count, cudaStream_t s,
                                  SearchProof proof = SearchProof {} );
-    void launch_bisector_validation( const CellContext & c, cudaStream_t s );
+    // warp per cell, over the listed cells or (null) all of the handle's
+    void launch_bisector_validation( const CellContext & c, const uint32_t * tasks, const uint32_t * count, cudaStream_t s );
 
     // Output extraction: per-cell owned counts, exclusive scans (totals[0] vertices,
     // totals[1] closed edges), then the writes bounded by the capacities.
@@ -265,4 +266,5 @@ namespace apo2
     void   spec_carve( SpecBuffers & b, void * base, uint32_t n );
     void   launch_edge_validation_speculative( const CellContext & c, const uint32_t * tasks, const uint32_t * task_count,
                                                const SpecBuffers & b, cudaStream_t s );
+    void   launch_bisector_validation_speculative( const CellContext & c, const SpecBuffers & b, cudaStream_t s );
 } // namespace apo2

@@ -44,11 +44,22 @@ namespace apo2
     // is long FP64 code, and run by one or two lanes at a time it held the warp for most
     // of its time.
     constexpr uint32_t kRefillAt = APO2_SPEC_REFILL_AT;
+#ifndef APO2_BISECTOR_REFILL_AT
+#define APO2_BISECTOR_REFILL_AT 24
+#endif
+#ifndef APO2_BISECTOR_STEPS
+#define APO2_BISECTOR_STEPS 8
+#endif
+    // the same for the bisectors, whose set-up is short, and the nodes a walk takes between two votes
+    constexpr uint32_t kBisectorRefillAt = APO2_BISECTOR_REFILL_AT;
+    constexpr uint32_t kBisectorSteps    = APO2_BISECTOR_STEPS;
 
     __device__ __forceinline__ uint32_t lane_of() { return threadIdx.x & 31; }
 
     // Sorted unique ids of a task cell's edge sites (the set the reference's known-neighbour
-    // and emptiness tests range over), and the cell's edge count for the item scan.
+    // and emptiness tests range over), and the cell's items for the item scan: its edges, or
+    // with Bisectors its neighbours of larger id (the tasks are then all cells of the handle).
+    template<bool Bisectors>
     __global__ void __launch_bounds__( kNbrBlock ) k_neighbor_lists( CellContext c, const uint32_t * __restrict__ tasks,
                                                                      const uint32_t * __restrict__ task_count,
                                                                      SpecBuffers b )
@@ -57,7 +68,7 @@ namespace apo2
         const uint32_t      warp  = threadIdx.x >> 5, lane = lane_of();
         const uint32_t      gwarp = blockIdx.x * ( kNbrBlock / 32 ) + warp;
         const uint32_t      nwarp = gridDim.x * ( kNbrBlock / 32 );
-        const uint32_t      count = *task_count;
+        const uint32_t      count = Bisectors ? c.hi - c.lo : *task_count;
         uint32_t *          ids   = buf[ warp ];
         for ( uint32_t t = gwarp; t < c.n; t += nwarp )
         {
@@ -67,12 +78,12 @@ namespace apo2
                     b.item_count[ t ] = 0;
                 continue;
             }
-            const uint32_t i  = tasks[ t ];
+            const uint32_t i  = Bisectors ? c.lo + t : tasks[ t ];
             const uint32_t en = c.edge_nb[ i ];
             const uint8_t  st = c.status[ i ];
-            if ( lane < kMaybeWords )
+            if ( !Bisectors && lane < kMaybeWords )
                 b.maybe_bits[ size_t( t ) * kMaybeWords + lane ] = 0;
-            if ( st == kFullyValidated || st == kBuried )
+            if ( ( !Bisectors && st == kFullyValidated ) || st == kBuried )
             {
                 if ( lane == 0 )
                 {
@@ -115,7 +126,7 @@ namespace apo2
                     }
                     __syncwarp();
                 }
-            uint32_t kept = 0, carried = kNone;
+            uint32_t kept = 0, above = 0, carried = kNone;
             for ( uint32_t base = 0; base < size; base += 32 )
             {
                 const uint32_t x    = base + lane;
@@ -130,15 +141,17 @@ namespace apo2
                 if ( keep && dst < kNbrCap )
                     b.nbr[ size_t( t ) * kNbrCap + dst ] = v;
                 kept += __popc( bal );
+                if ( Bisectors )
+                    above += __popc( __ballot_sync( 0xffffffffu, keep && v > i && v < c.n ) );
             }
             __syncwarp();
-            if ( kept > kNbrCap && lane < kMaybeWords )
+            if ( !Bisectors && kept > kNbrCap && lane < kMaybeWords )
                 b.maybe_bits[ size_t( t ) * kMaybeWords + lane ] = 0xffffffffu; // nothing decided: full exact pass
             if ( lane == 0 )
             {
                 b.nbr_count[ t ]  = min( kept, kNbrCap );
                 b.cell_flag[ t ]  = kept > kNbrCap ? kFlagOverflow : 0u;
-                b.item_count[ t ] = kept > kNbrCap ? 0u : en;
+                b.item_count[ t ] = kept > kNbrCap ? 0u : ( Bisectors ? above : en );
             }
         }
     }
@@ -692,6 +705,220 @@ namespace apo2
         }
     }
 
+    // -----------------------------------------------------------------------------------
+    // Bisector validation as a search over all (cell, neighbour) pairs, with the warp-per-cell pass
+    // (k_bisector_validation) for the cells where one found a site
+    // -----------------------------------------------------------------------------------
+    // A bisector (i, k) is searched for a site inside the cylinder between its two spheres that would
+    // close a trisector on it (algorithm.inl:859-1233). Hardly any is found, and while none is the
+    // cell stays as it is, so as for the edges only existence matters and the pairs of all cells are
+    // independent: each is one lane's item. The warp-per-cell pass had a cell's 7 or so neighbours of
+    // larger id on 32 lanes, 150 registers and its cell in shared memory for each such walk; bound by
+    // the latency of dependent node loads, which 64 registers and full warps hide far better. With
+    // the pruned entry below: 1M-site protein packing 67.6 -> 7.5 ms (2.5 of it the neighbour
+    // lists), 1M log-normal cloud 97 -> 30 ms (5.9 in the exact pass), 61k protein 13.1 -> 0.6 ms
+    // (one cell's walk), 46^3 lattice 4.7 -> 0.5 ms.
+    struct BisectorSearch
+    {
+        uint32_t t, i, k;
+        float3   fci, fck;
+        float4   bsph;     // the ball that must hold the site
+        float    cylinder; // and the radius of the cylinder around the axis
+        // entering a box: the site's sphere lies in the ball, so a box at a distance has to reach at
+        // least a smallest sphere's diameter (`shrink`, less a rounding margin) into it; and it
+        // lies in the cylinder, so the box has to come within `tube` of the axis
+        float3   axis;
+        float    shrink, tube, slack;
+    };
+
+    // Sets up the search of pair (i, k); false when the security radius covers it.
+    __device__ __forceinline__ bool setup_bisector( const CellContext & c, BisectorSearch & s, float known )
+    {
+        const float4 si = c.sites_f[ s.i ], sk = c.sites_f[ s.k ];
+        s.fci = f3( si );
+        s.fck = f3( sk );
+        if ( lt_eps( flength( s.fci - s.fck ) + si.w + sk.w, known ) )
+            return false;
+        const float3 center = ( s.fci + s.fck ) * .5f;
+        const float  radius = flength( center - s.fci ) + fmaxf( si.w, sk.w );
+        s.bsph              = make_float4( center.x, center.y, center.z, radius );
+        s.cylinder          = fmaxf( si.w, sk.w );
+        // Margins: the leaf's containment test rounds within 4e-7 of the radius, boxes and centre
+        // within 2e-7 of the coordinates; the distance from the axis is a root of a difference
+        // of squares that are off by 1.1e-6 of the squared distance from c_i, at most twice the
+        // radius. Each is taken several times over.
+        const float diameter = 2.f * fmaxf( 0.f, float( c.scene->rmin ) );
+        const float reach    = 4e-6f * ( fabsf( center.x ) + fabsf( center.y ) + fabsf( center.z ) + radius );
+        s.shrink             = fmaxf( 0.f, diameter - reach );
+        s.slack              = 5e-6f;
+        s.tube               = s.cylinder - s.shrink + fmaxf( 0.f, -float( c.scene->rmin ) ) + 6e-3f * radius + reach;
+        s.axis               = fnormalize( s.fck - s.fci );
+        return true;
+    }
+
+    __device__ __forceinline__ bool enter_child( const BisectorSearch & s, const Box & b )
+    {
+        const float d = b.distance( s.bsph );
+        // -radius: the centre is inside the box
+        if ( !( d < 0.f ) || !( d < -s.shrink || d == -s.bsph.w ) )
+            return false;
+        const float3 half = ( b.hi - b.lo ) * .5f;
+        const float3 from = ( b.lo + b.hi ) * .5f - s.fci;
+        const float  v    = fdot( from, s.axis ), ff = fdot( from, from );
+        const float  r    = s.tube + flength( half ) * 1.0001f;
+        return !( ff - v * v - s.slack * ff > r * r ); // r > 0; NaN enters
+    }
+
+    __device__ __forceinline__ bool closes_trisector( const CellContext & c, const SpecBuffers & b, const BisectorSearch & s, uint32_t j )
+    {
+        if ( j == s.i || j == s.k )
+            return false;
+        const float4 fj = c.sites_f[ j ];
+        const float3 cj = f3( fj );
+        if ( !( s.bsph.w >= fj.w && ( flength( f3( s.bsph ) - cj ) <= ( s.bsph.w - fj.w ) ) ) )
+            return false;
+        const float3 itoj = cj - s.fci;
+        const float  v    = fdot( itoj, s.axis );
+        const float  d    = sqrtf( fdot( itoj, itoj ) - v * v );
+        if ( !( ( d + fj.w ) < s.cylinder ) )
+            return false;
+        const uint32_t * nbr   = b.nbr + size_t( s.t ) * kNbrCap;
+        const uint32_t   count = b.nbr_count[ s.t ];
+        if ( in_sorted( nbr, count, j ) )
+            return false;
+        double4 x0 = make_double4( 0, 0, 0, 0 ), x1 = make_double4( 0, 0, 0, 0 );
+        if ( trisector( c.sites[ s.i ], c.sites[ j ], c.sites[ s.k ], x0, x1 ) != 2 )
+            return false;
+        FilterTally untallied;
+        for ( uint32_t q = 0; q < count; q++ )
+            if ( nbr[ q ] != s.k
+                 && ( c.fp32 ? site_conflict<true>( c, nbr[ q ], x1, untallied ) : site_conflict<false>( c, nbr[ q ], x1, untallied ) ) )
+                return false;
+        return true;
+    }
+
+    __global__ void __launch_bounds__( kSpecBlock, 8 ) k_bisector_speculate( CellContext c, SpecBuffers b )
+    {
+        const uint32_t count = c.hi - c.lo;
+        const uint64_t total = *b.item_total;
+        const uint32_t n     = c.n;
+        uint32_t       err   = 0;
+
+        BisectorSearch s;
+        bool           active = false, exhausted = false;
+        uint32_t       stack[ kStack ];
+        int            sp   = 0;
+        uint32_t       node = 0;
+        while ( true )
+        {
+            const uint32_t idle = __ballot_sync( 0xffffffffu, !active && !exhausted );
+            const uint32_t busy = __ballot_sync( 0xffffffffu, active );
+            if ( idle == 0 && busy == 0 )
+                break;
+            if ( idle != 0 && ( busy == 0 || uint32_t( __popc( idle ) ) >= kBisectorRefillAt ) )
+            {
+                if ( !active && !exhausted )
+                {
+                    const uint32_t leader = __ffs( idle ) - 1;
+                    uint64_t       base   = 0;
+                    if ( lane_of() == leader )
+                        base = atomicAdd( reinterpret_cast<unsigned long long *>( b.item_counter ), __popc( idle ) );
+                    base                = __shfl_sync( idle, base, leader );
+                    const uint64_t item = base + __popc( idle & ( ( 1u << lane_of() ) - 1u ) );
+                    if ( item >= total )
+                        exhausted = true;
+                    else
+                    {
+                        uint32_t lo = 0, hi = count;
+                        while ( hi - lo > 1 )
+                        {
+                            const uint32_t mid = ( lo + hi ) >> 1;
+                            if ( b.item_offset[ mid ] <= item )
+                                lo = mid;
+                            else
+                                hi = mid;
+                        }
+                        s.t = lo;
+                        s.i = c.lo + lo;
+                        // the item's place among the sorted neighbours, counted from the first above i
+                        const uint32_t * nbr   = b.nbr + size_t( s.t ) * kNbrCap;
+                        uint32_t         first = 0, last = b.nbr_count[ s.t ];
+                        while ( first < last )
+                        {
+                            const uint32_t mid = ( first + last ) >> 1;
+                            if ( nbr[ mid ] <= s.i )
+                                first = mid + 1;
+                            else
+                                last = mid;
+                        }
+                        s.k = nbr[ first + uint32_t( item - b.item_offset[ s.t ] ) ];
+                        if ( setup_bisector( c, s, c.known_radii[ s.i ] ) )
+                        {
+                            active = true;
+                            sp     = 0;
+                            node   = 0;
+                        }
+                    }
+                }
+                continue;
+            }
+            // some nodes of every walk between two votes; the leaf children of a node are tested with it
+#pragma unroll 1
+            for ( uint32_t step = 0; step < kBisectorSteps && active; step++ )
+            {
+                Box      lb, rb;
+                uint32_t lc, rc;
+                load_node( c.nodes, node, lb, rb, lc, rc );
+                const bool eL = enter_child( s, lb ), eR = enter_child( s, rb );
+                uint32_t   next = kNone;
+                bool       hit  = false;
+                if ( eL )
+                {
+                    if ( lc >= n - 1 )
+                        hit = closes_trisector( c, b, s, lc - ( n - 1 ) );
+                    else
+                        next = lc;
+                }
+                if ( eR && !hit )
+                {
+                    if ( rc >= n - 1 )
+                        hit = closes_trisector( c, b, s, rc - ( n - 1 ) );
+                    else if ( next == kNone )
+                        next = rc;
+                    else if ( sp < int( kStack ) )
+                        stack[ sp++ ] = rc;
+                    else
+                        err |= kErrStack;
+                }
+                if ( hit )
+                {
+                    atomicOr( &b.cell_flag[ s.t ], kFlagFound );
+                    active = false;
+                }
+                else if ( next != kNone )
+                    node = next;
+                else if ( sp > 0 )
+                    node = stack[ --sp ];
+                else
+                    active = false;
+            }
+        }
+        if ( err )
+            atomicOr( c.error, err );
+    }
+
+    // Cells where no bisector found a site are validated; the others are listed for the exact pass.
+    __global__ void k_bisector_commit( CellContext c, SpecBuffers b )
+    {
+        const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+        if ( t >= c.hi - c.lo || c.status[ c.lo + t ] == kBuried )
+            return;
+        if ( b.cell_flag[ t ] )
+            b.exact_tasks[ atomicAdd( b.exact_count, 1u ) ] = c.lo + t;
+        else
+            c.status[ c.lo + t ] = kFullyValidated;
+    }
+
     // long lane searches per round: log-normal radii reach 1.5 per site
     static size_t heavy_capacity( uint32_t n ) { return 6 * size_t( n ) + 65536; }
     static size_t sub_capacity( uint32_t n ) { return 4 * size_t( n ) + 65536; }
@@ -756,7 +983,7 @@ namespace apo2
 
     // Persistent grid sizes per device (148 SMs x resident blocks of each kernel on B200).
     constexpr int        kSpecDevices = 64;
-    static int           g_spec_grid[ kSpecDevices ], g_heavy_grid[ kSpecDevices ];
+    static int           g_spec_grid[ kSpecDevices ], g_heavy_grid[ kSpecDevices ], g_bisector_grid[ kSpecDevices ];
     static PerDeviceOnce g_spec_config;
 
     static int spec_device()
@@ -778,6 +1005,8 @@ namespace apo2
             g_spec_grid[ dev ] = sms * std::max( 1, per_sm );
             cudaOccupancyMaxActiveBlocksPerMultiprocessor( &per_sm, k_edge_heavy, kHeavyBlock, 0 );
             g_heavy_grid[ dev ] = sms * std::max( 1, per_sm );
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor( &per_sm, k_bisector_speculate, kSpecBlock, 0 );
+            g_bisector_grid[ dev ] = sms * std::max( 1, per_sm );
         } );
     }
 
@@ -789,7 +1018,7 @@ namespace apo2
         const int spec_grid  = dev >= 0 ? g_spec_grid[ dev ] : 148 * 4; // an ordinal outside the table
         const int heavy_grid = dev >= 0 ? g_heavy_grid[ dev ] : 148 * 4;
         const uint32_t nbr_blocks = std::max( 1u, std::min<uint32_t>( ( c.n + 3 ) / 4, 148 * 32 ) );
-        APO2_LAUNCH( "k_neighbor_lists", s, k_neighbor_lists<<<nbr_blocks, kNbrBlock, 0, s>>>( c, tasks, task_count, b ) );
+        APO2_LAUNCH( "k_neighbor_lists", s, k_neighbor_lists<false><<<nbr_blocks, kNbrBlock, 0, s>>>( c, tasks, task_count, b ) );
         scan_exclusive( b.item_count, c.n, b.scan_sums, b.item_total, s );
         cudaMemsetAsync( b.item_counter, 0, sizeof( uint64_t ), s );
         cudaMemsetAsync( b.exact_count, 0, sizeof( uint32_t ), s );
@@ -808,5 +1037,21 @@ namespace apo2
         proof.nbr        = b.nbr;
         proof.nbr_count  = b.nbr_count;
         launch_edge_validation( c, b.exact_tasks, b.exact_count, s, proof );
+    }
+
+    void launch_bisector_validation_speculative( const CellContext & c, const SpecBuffers & b, cudaStream_t s )
+    {
+        configure_spec_kernels();
+        const int      dev        = spec_device();
+        const int      grid       = dev >= 0 ? g_bisector_grid[ dev ] : 148 * 8; // an ordinal outside the table
+        const uint32_t cells      = c.hi - c.lo;
+        const uint32_t nbr_blocks = std::max( 1u, std::min<uint32_t>( ( c.n + 3 ) / 4, 148 * 32 ) );
+        APO2_LAUNCH( "k_neighbor_lists", s, k_neighbor_lists<true><<<nbr_blocks, kNbrBlock, 0, s>>>( c, nullptr, nullptr, b ) );
+        scan_exclusive( b.item_count, c.n, b.scan_sums, b.item_total, s );
+        cudaMemsetAsync( b.item_counter, 0, sizeof( uint64_t ), s );
+        cudaMemsetAsync( b.exact_count, 0, sizeof( uint32_t ), s );
+        APO2_LAUNCH( "k_bisector_speculate", s, k_bisector_speculate<<<grid, kSpecBlock, 0, s>>>( c, b ) );
+        APO2_LAUNCH( "k_bisector_commit", s, k_bisector_commit<<<std::max( 1u, ( cells + 255 ) / 256 ), 256, 0, s>>>( c, b ) );
+        launch_bisector_validation( c, b.exact_tasks, b.exact_count, s );
     }
 } // namespace apo2
