@@ -409,7 +409,7 @@ namespace
         total += align256( 4 * size_t( n ) ) * 2 + align256( 4 * scanWords * 2 ) + align256( 16 );
         total += align256( spec_bytes( n ) );
         total += align256( walk_scratch_bytes() ) + align256( 4 );
-        total += align256( sizeof( unsigned long long ) * kCounters );
+        total += align256( sizeof( unsigned long long ) * kCounters ) + align256( 4 * size_t( n ) ) + align256( 8 * size_t( n ) );
         return total;
     }
 
@@ -472,6 +472,8 @@ namespace
         c.walk_scratch    = a.take<uint32_t>( walk_scratch_bytes() / sizeof( uint32_t ) );
         c.work_counter    = a.take<uint32_t>( 1 );
         c.counters        = a.take<unsigned long long>( kCounters );
+        c.largest         = a.take<float>( n );
+        c.around          = a.take<uint2>( n );
         c.fp32            = opt.precision == APO2_PRECISION_FP32_FILTER ? 1u : 0u;
         c.codes           = t.codes;
         sort_scratch_carve( h->sort, sortBase, n, h->error );

@@ -690,6 +690,19 @@ namespace apo2
         return written != 0;
     }
 
+    // Largest vertex radius of the cell, at least 0.
+    template<class W>
+    __device__ __forceinline__ double largest_radius( const W & w )
+    {
+        double m = 0.0;
+        for ( uint32_t v = lane_id(); v < w.vn; v += 32 )
+            m = fmax( m, w.pos[ v ].w );
+#pragma unroll
+        for ( int o = 16; o > 0; o >>= 1 )
+            m = fmax( m, __shfl_xor_sync( kFull, m, o ) );
+        return m;
+    }
+
     // Largest vertex or closed-trisector radius of the cell (topology_update.inl:595-653).
     template<class W>
     __device__ double cell_radius( const CellContext & c, const W & w, double4 si )
@@ -1248,6 +1261,11 @@ namespace apo2
             const double4 si = c.sites[ i ];
             load_cell( c, w, i, si, true, true );
             const float known = c.known_radii[ i ];
+            // the walks of the first pass start at the node around everything that the cell's spheres
+            // come near to
+            float4 field = touch_ball( c, si, largest_radius( w ) );
+            field.w += 2e-2f + 2e-5f * ( fabsf( field.x ) + fabsf( field.y ) + fabsf( field.z ) + field.w );
+            const uint32_t start = node_around( c.nodes, n, field );
 
             uint32_t vs = 0, restarts = 0;
             while ( vs < w.vn / 32 + 1 && restarts < 100 )
@@ -1295,7 +1313,7 @@ namespace apo2
                 {
                     uint2    stack[ kStack ];
                     int      sp         = 0;
-                    uint32_t node       = 0;
+                    uint32_t node       = pass == 0 && 2.f * fmaxf( fc.w, 0.f ) + float( si.w ) + bound <= field.w ? start : 0u;
                     float    best       = pass == 0 ? bound : FLT_MAX;
                     bool     walking    = searching;
                     uint32_t walk_steps = 0;
@@ -1399,6 +1417,17 @@ namespace apo2
                 }
             }
             store_cell( c, w, i, 0, err );
+            // for the edge searches
+            const double last  = largest_radius( w );
+            const float4 touch = touch_ball( c, si, last );
+            uint2        around;
+            around.y = node_around( c.nodes, n, make_float4( touch.x, touch.y, touch.z, touch.w + 1.001f * float( c.scene->rmax - c.scene->rmin ) ) );
+            around.x = node_around( c.nodes, n, touch, around.y );
+            if ( lane == 0 )
+            {
+                c.largest[ i ] = float( last );
+                c.around[ i ]  = around;
+            }
             __syncwarp();
         }
         report( c, err, w );
@@ -1417,8 +1446,9 @@ namespace apo2
     // trisector and the ball its contributors must reach (see k_edge_validation).
     struct EdgeWalk
     {
-        float4   bsph, reach;
-        float3   n1, n2, pp1, pp2;
+        float4    bsph;
+        EdgeReach reach;
+        TangentPlanes planes;
         bool     hyperbola;
         uint32_t k, l;
         double4  sk, sl;
@@ -1468,12 +1498,12 @@ namespace apo2
             const uint32_t farChild = leftClosest ? rc : lc, closeChild = leftClosest ? lc : rc;
             bool           exploreFar = minFar < 0.f;
             if ( p.hyperbola && exploreFar )
-                exploreFar = fdot( p.n1, farPoint - p.pp1 ) < 0.f && fdot( p.n2, farPoint - p.pp2 ) < 0.f;
+                exploreFar = fdot( p.planes.n1, farPoint - p.planes.p1 ) < 0.f && fdot( p.planes.n2, farPoint - p.planes.p2 ) < 0.f;
             bool exploreClose = minClose < 0.f;
             if ( p.hyperbola && exploreClose )
-                exploreClose = fdot( p.n1, closePoint - p.pp1 ) < 0.f && fdot( p.n2, closePoint - p.pp2 ) < 0.f;
-            exploreFar   = exploreFar && ( leftClosest ? rb : lb ).distance( p.reach ) < 0.f;
-            exploreClose = exploreClose && ( leftClosest ? lb : rb ).distance( p.reach ) < 0.f;
+                exploreClose = fdot( p.planes.n1, closePoint - p.planes.p1 ) < 0.f && fdot( p.planes.n2, closePoint - p.planes.p2 ) < 0.f;
+            exploreFar   = exploreFar && within( p.reach, p.planes, leftClosest ? rb : lb );
+            exploreClose = exploreClose && within( p.reach, p.planes, leftClosest ? lb : rb );
             if ( exploreClose )
             {
                 first = closeChild;
@@ -1499,10 +1529,10 @@ namespace apo2
             {
                 sj              = c.sites[ j ];
                 const float4 fj = to_float( sj );
-                can             = intersects( fj, p.bsph ) && flength( f3( fj ) - f3( p.reach ) ) <= p.reach.w;
+                can             = intersects( fj, p.bsph ) && within( p.reach, p.planes, fj );
                 if ( p.hyperbola )
-                    can = can && double( fdot( p.n1, f3( fj ) - p.pp1 ) ) < -sj.w
-                          && double( fdot( p.n2, f3( fj ) - p.pp2 ) ) < -sj.w;
+                    can = can && double( fdot( p.planes.n1, f3( fj ) - p.planes.p1 ) ) < -sj.w
+                          && double( fdot( p.planes.n2, f3( fj ) - p.planes.p2 ) ) < -sj.w;
             }
             if ( can )
                 can = !known_by_lane( w, j );
@@ -1674,8 +1704,7 @@ namespace apo2
                 }
                 const bool   hyperbola = type == 1, ellipse = type == 2;
                 const float4 v1 = to_float( ev0 ), v2 = to_float( ev1 );
-                float3       n1 = make_float3( 0, 0, 0 ), n2 = make_float3( 0, 0, 0 );
-                float3       pp1 = make_float3( 0, 0, 0 ), pp2 = make_float3( 0, 0, 0 );
+                TangentPlanes planes {};
                 float4       bsph = make_float4( 0, 0, 0, 0 );
                 if ( need && ellipse )
                 {
@@ -1687,16 +1716,16 @@ namespace apo2
                 {
                     double3 nn1, nn2;
                     tangent_planes( si, sk, sl, nn1, nn2 );
-                    n1               = to_float( nn1 );
-                    n2               = to_float( nn2 );
+                    planes.n1        = to_float( nn1 );
+                    planes.n2        = to_float( nn2 );
                     const double3 p1 = d3( si ) + nn1 * si.w;
                     const double3 p2 = d3( sk ) + nn1 * sk.w;
                     const double3 p3 = d3( sl ) + nn1 * sl.w;
                     const double3 p4 = d3( si ) + nn2 * si.w;
                     const double3 p5 = d3( sk ) + nn2 * sk.w;
                     bsph             = to_float( sphere_from_points( p1, p2, p3, p5 ) );
-                    pp1              = to_float( p1 );
-                    pp2              = to_float( p4 );
+                    planes.p1        = to_float( p1 );
+                    planes.p2        = to_float( p4 );
                 }
                 const bool inside = lt_eps( flength( f3( fsi ) - f3( bsph ) ), known - bsph.w );
                 if ( eid < w.en && inside )
@@ -1704,33 +1733,24 @@ namespace apo2
                     w.e[ eid ].w = ( w.e[ eid ].w & 0xffffff00u ) | 1u;
                     need         = false;
                 }
-                // reach of the search (see reach_radius): the stored vertices and the ones
+                // reach of the search (see EdgeReach): the stored vertices and the ones
                 // added by this pass that lie on the edge, and its possible apexes
-                float4 reach = make_float4( fsi.x, fsi.y, fsi.z, 0.f );
+                EdgeReach reach {};
                 // the third sites of the stored vertices on this edge: the neighbours bounding its
                 // arc, tested first against a candidate root while the cell is the stored one
                 // (whose vertex sites are all edge sites, so they belong to the same conjunction)
-                uint32_t hint0 = kNone, hint1 = kNone;
+                uint32_t hint[ 2 ] = { kNone, kNone };
                 if ( need )
                 {
-                    double         wmax = 0.0;
-                    const uint32_t svn  = c.vertex_nb[ i ];
-                    for ( uint32_t v = 0; v < svn; v++ )
-                    {
-                        const uint4 r = c.vertices[ store_row( c, i ) * kMaxVertices + v ];
-                        if ( vertex_on_edge( r, k, l ) )
-                        {
-                            wmax             = fmax( wmax, solve_vertex( c, si, r ).w );
-                            const uint32_t m = ( r.x != k && r.x != l ) ? r.x : ( ( r.y != k && r.y != l ) ? r.y : r.z );
-                            if ( hint0 == kNone )
-                                hint0 = m;
-                            else if ( hint1 == kNone && m != hint0 )
-                                hint1 = m;
-                        }
-                    }
+                    ArcEnds ends;
+                    double  wmax = stored_ends( c, i, si, k, l, ends, hint );
                     for ( uint32_t v = 0; v < w.vn; v++ )
                         if ( vertex_on_edge( w.v[ v ], k, l ) )
-                            wmax = fmax( wmax, w.pos[ v ].w );
+                        {
+                            const uint4 r = w.v[ v ];
+                            wmax          = fmax( wmax, w.pos[ v ].w );
+                            ends.add( w.pos[ v ], third_site( r, k, l ) );
+                        }
                     if ( ellipse || cnt == kNone )
                     {
                         const double4 apex[ 2 ] = { ev0, ev1 };
@@ -1749,7 +1769,7 @@ namespace apo2
                                 wmax = fmax( wmax, apex[ a ].w );
                         }
                     }
-                    reach.w = reach_radius( wmax, si.w, c.scene->rmax );
+                    reach = edge_reach( c, si, sk, sl, hyperbola, ends, wmax, bsph );
                 }
 
                 // proven free of contributors on this very cell state
@@ -1808,12 +1828,12 @@ namespace apo2
                         const uint32_t farChild = leftClosest ? rc : lc, closeChild = leftClosest ? lc : rc;
                         bool           exploreFar = minFar < 0.f;
                         if ( hyperbola && exploreFar )
-                            exploreFar = fdot( n1, farPoint - pp1 ) < 0.f && fdot( n2, farPoint - pp2 ) < 0.f;
+                            exploreFar = fdot( planes.n1, farPoint - planes.p1 ) < 0.f && fdot( planes.n2, farPoint - planes.p2 ) < 0.f;
                         bool exploreClose = minClose < 0.f;
                         if ( hyperbola && exploreClose )
-                            exploreClose = fdot( n1, closePoint - pp1 ) < 0.f && fdot( n2, closePoint - pp2 ) < 0.f;
-                        exploreFar   = exploreFar && ( leftClosest ? rb : lb ).distance( reach ) < 0.f;
-                        exploreClose = exploreClose && ( leftClosest ? lb : rb ).distance( reach ) < 0.f;
+                            exploreClose = fdot( planes.n1, closePoint - planes.p1 ) < 0.f && fdot( planes.n2, closePoint - planes.p2 ) < 0.f;
+                        exploreFar   = exploreFar && within( reach, planes, leftClosest ? rb : lb );
+                        exploreClose = exploreClose && within( reach, planes, leftClosest ? lb : rb );
                         if ( !exploreFar && !exploreClose )
                             break;
                         node = exploreClose ? closeChild : farChild;
@@ -1833,10 +1853,10 @@ namespace apo2
                     {
                         sj              = c.sites[ j ];
                         const float4 fj = to_float( sj );
-                        can             = intersects( fj, bsph ) && flength( f3( fj ) - f3( reach ) ) <= reach.w;
+                        can             = intersects( fj, bsph ) && within( reach, planes, fj );
                         if ( hyperbola )
-                            can = can && double( fdot( n1, f3( fj ) - pp1 ) ) < -sj.w
-                                  && double( fdot( n2, f3( fj ) - pp2 ) ) < -sj.w;
+                            can = can && double( fdot( planes.n1, f3( fj ) - planes.p1 ) ) < -sj.w
+                                  && double( fdot( planes.n2, f3( fj ) - planes.p2 ) ) < -sj.w;
                     }
                     uint32_t cm = __ballot_sync( kFull, can );
                     while ( cm )
@@ -1869,7 +1889,7 @@ namespace apo2
                             const uint32_t nv = __ffs( tm ) - 1;
                             tm &= ~( 1u << nv );
                             const double4  cand = shfl4( nv ? x1 : x0, t2 );
-                            const uint32_t h0 = __shfl_sync( kFull, hint0, t2 ), h1 = __shfl_sync( kFull, hint1, t2 );
+                            const uint32_t h0 = __shfl_sync( kFull, hint[ 0 ], t2 ), h1 = __shfl_sync( kFull, hint[ 1 ], t2 );
                             const bool     hinted = pristine && ( ( h0 != kNone && site_conflict<Fp32>( c, h0, cand, w.tally ) )
                                                               || ( h1 != kNone && site_conflict<Fp32>( c, h1, cand, w.tally ) ) );
                             const bool     ok   = !hinted && edges_clear( c, w, cand, tk, tl );
@@ -1900,11 +1920,19 @@ namespace apo2
                     pending &= pending - 1;
                     EdgeWalk p;
                     p.bsph      = shfl4f( bsph, src );
-                    p.reach     = shfl4f( reach, src );
-                    p.n1        = shfl3( n1, src );
-                    p.n2        = shfl3( n2, src );
-                    p.pp1       = shfl3( pp1, src );
-                    p.pp2       = shfl3( pp2, src );
+                    for ( int q = 0; q < 3; q++ )
+                        p.reach.ball[ q ] = shfl4f( reach.ball[ q ], src );
+                    for ( int q = 0; q < 2; q++ )
+                        p.reach.slab[ q ] = __shfl_sync( kFull, reach.slab[ q ], src );
+                    p.reach.limit = shfl4f( reach.limit, src );
+                    p.reach.kind  = __shfl_sync( kFull, reach.kind, src );
+                    p.reach.diameter = __shfl_sync( kFull, reach.diameter, src );
+                    p.reach.margin   = __shfl_sync( kFull, reach.margin, src );
+                    p.reach.below    = __shfl_sync( kFull, int( reach.below ), src ) != 0;
+                    p.planes.n1        = shfl3( planes.n1, src );
+                    p.planes.n2        = shfl3( planes.n2, src );
+                    p.planes.p1       = shfl3( planes.p1, src );
+                    p.planes.p2       = shfl3( planes.p2, src );
                     p.hyperbola = __shfl_sync( kFull, int( hyperbola ), src ) != 0;
                     p.k         = __shfl_sync( kFull, k, src );
                     p.l         = __shfl_sync( kFull, l, src );

@@ -48,6 +48,11 @@ namespace apo2
         const Scene *    scene       = nullptr; // bounds and radius range of the sites
         uint32_t *       walk_scratch = nullptr; // kWalkScratchWords per warp of the exact edge pass
         uint32_t *       work_counter = nullptr; // next cell of the dynamically scheduled passes
+        // left by the vertex validation for the edge searches of the same round: the largest vertex
+        // radius of each cell, and the nodes around everything that its spheres can touch (x) and
+        // around everything within the general bound of its edges (y)
+        float * largest = nullptr;
+        uint2 * around  = nullptr;
         // learned k-proposal (null: the plain form): the network, the Morton codes its features
         // read, and the proposed rank of every site (written by the first kNN step)
         const ProposalNet * proposal   = nullptr;
@@ -143,15 +148,310 @@ namespace apo2
     // the edge's arc inside the current cell, whose empty-sphere radius w(x) is at most the
     // largest radius over the arc: its vertices and, on an elliptic trisector, an apex that
     // may lie on the arc (the cell certificate of the reference rests on the same bound,
-    // algorithm.inl:186-190, topology_update.inl:595-653). Then
-    //     |c_j - c_i| <= |c_j - x| + |x - c_i| = 2 w(x) + r_i + r_j,
-    // so the search may skip every BVH node and leaf outside that ball: the leaves it
-    // visits are a subsequence of the reference's, in the same order, and every site that
-    // could contribute is among them, so the first contributor found is the same.
+    // algorithm.inl:186-190, topology_update.inl:595-653). Sphere j touches the sphere of radius
+    // w(x) around x, so the search may skip every BVH node and leaf away from all such spheres: the
+    // leaves it visits are a subsequence of the reference's, in the same order, and every site
+    // that could contribute is among them, so the first contributor found is the same.
+    //
+    // That bound is kReachBall: one ball around c_i, |c_j - c_i| <= 2 w + r_i + r_max, or the
+    // reference's own bounding sphere where that is smaller. Between two vertices the spheres along
+    // the arc lie in three far smaller balls (arc_reach).
+    //
+    // One kind of contributor lies outside them: a root so far away that the single-precision
+    // lengths of the emptiness test cannot tell the neighbours apart (its radius is 7e7 and more
+    // where it happened, once in some ten builds, on edges of hull cells). The reference
+    // takes such a root, so it has to be found. It belongs to a site that touches a plane tangent to
+    // the edge's three sites, so on a hyperbolic trisector the boxes that reach one of the two planes
+    // within the general bound are entered too (kReachArcPlanes); an elliptic one has no
+    // point further than its apex. Most planes are out, though (far_roots_blocked).
     // ---------------------------------------------------------------------------------
+    constexpr uint32_t kReachBall = 0, kReachArc = 1, kReachArcPlanes = 2;
+    constexpr double   kFarRoot   = 2.5e5; // radius from which a root counts as far: single precision is off by 0.1 there
+
+    struct EdgeReach
+    {
+        float4   ball[ 3 ]; // kReachBall: the same one three times
+        float4   limit;     // kReachArcPlanes: ball holding every site that the planes let in
+        float    slab[ 2 ]; // and how near to each plane it has to come
+        // hyperbolic trisectors: a contributor lies wholly below both planes (algorithm.inl:695-700), so
+        // a box has to go below them by a smallest sphere's diameter; less this rounding margin
+        float    diameter, margin;
+        bool     below;
+        uint32_t kind;
+    };
+    struct TangentPlanes
+    {
+        float3 n1, n2, p1, p2;
+    };
+
+    __device__ __forceinline__ bool meets( float4 ball, const Box & b )
+    {
+        const float3 d = f3( ball ) - b.closest( ball );
+        return fdot( d, d ) <= ball.w * ball.w;
+    }
+    __device__ __forceinline__ bool meets( float4 ball, float4 site )
+    {
+        const float3 d = f3( ball ) - f3( site );
+        const float  r = ball.w + site.w;
+        return ( r >= 0.f ) & ( fdot( d, d ) <= r * r );
+    }
+    // Heights over a plane: .x, negative if something of the box or the sphere can be wholly below,
+    // and .y of its highest point.
+    __device__ __forceinline__ float2 heights( float3 n, float3 p, float diameter, const Box & b )
+    {
+        const float3 m = ( b.lo + b.hi ) * .5f - p, h = ( b.hi - b.lo ) * .5f;
+        const float  s = fdot( n, m ), e = fabsf( n.x ) * h.x + fabsf( n.y ) * h.y + fabsf( n.z ) * h.z;
+        return make_float2( s - e + diameter, s + e );
+    }
+    __device__ __forceinline__ float2 heights( float3 n, float3 p, float, float4 site )
+    {
+        const float top = fdot( n, f3( site ) - p ) + site.w;
+        return make_float2( top, top );
+    }
+    // The sphere of a leaf from its box, which was made from it: the rounding of the box's corners
+    // is in the radius.
+    __device__ __forceinline__ float4 sphere_in( const Box & b )
+    {
+        const float3 m = ( b.lo + b.hi ) * .5f;
+        const float  r = fmaxf( fmaxf( b.hi.x - b.lo.x, b.hi.y - b.lo.y ), b.hi.z - b.lo.z ) * .5f;
+        return make_float4( m.x, m.y, m.z, r + 1e-6f * ( fabsf( m.x ) + fabsf( m.y ) + fabsf( m.z ) + fabsf( r ) ) );
+    }
+    // May box or site `x` be, or hold, a contributor? The balls are tested without branches: a walk's
+    // lanes would take them all the same.
+    template<class X>
+    __device__ __forceinline__ bool within( const EdgeReach & a, const TangentPlanes & t, const X & x )
+    {
+        bool in = meets( a.ball[ 0 ], x ) | meets( a.ball[ 1 ], x ) | meets( a.ball[ 2 ], x );
+        if ( a.below )
+        {
+            const float2 h1 = heights( t.n1, t.p1, a.diameter, x ), h2 = heights( t.n2, t.p2, a.diameter, x );
+            if ( a.kind == kReachArcPlanes )
+                in = in | ( ( ( h1.y >= -a.slab[ 0 ] ) | ( h2.y >= -a.slab[ 1 ] ) ) & meets( a.limit, x ) );
+            in = in & ( h1.x < a.margin ) & ( h2.x < a.margin );
+        }
+        return in;
+    }
+
+    // Does neighbour m conflict with every far root beyond the plane of outward normal n? Its
+    // distance to the root and that of c_i, taken from the same far point, are rounded to single
+    // precision alike: where m is the nearer one it does not come out farther, and the test of m
+    // against the root's radius, re-measured from c_i, is decided by the larger radius of m. (The
+    // approximate root falls between neighbouring floats at 508 of the 2^31 positive ones.)
+    __device__ __forceinline__ bool far_roots_blocked( float3 n, float4 fi, float4 m )
+    {
+        const float3 e  = f3( m ) - f3( fi );
+        const float  ee = fdot( e, e );
+        return m.w >= fi.w + 1e-3f && fdot( n, e ) >= 5e-3f * sqrtf( ee ) + float( 1.0 / kFarRoot ) * ee;
+    }
+
+    // The ball with its margins: 1 % and 1e-3 as the reach always had, and the rounding of a far
+    // centre to float.
+    __device__ __forceinline__ float4 reach_ball( double3 x, double r )
+    {
+        r = fmax( r, 0.0 );
+        r = r * 1.01 + 1e-3 * ( 1.0 + r ) + 1e-6 * ( fabs( x.x ) + fabs( x.y ) + fabs( x.z ) );
+        return make_float4( float( x.x ), float( x.y ), float( x.z ), float( r ) );
+    }
+
     __device__ __forceinline__ bool vertex_on_edge( uint4 r, uint32_t k, uint32_t l )
     {
         return ( r.x == k || r.y == k || r.z == k ) && ( r.x == l || r.y == l || r.z == l );
+    }
+
+    // Ends of an edge's arc: its two vertices and the third site of each.
+    struct ArcEnds
+    {
+        double4  v[ 2 ];
+        uint32_t m[ 2 ];
+        uint32_t count = 0; // stored vertices on the edge
+        __device__ __forceinline__ void add( double4 x, uint32_t site )
+        {
+            if ( count < 2 )
+            {
+                ( count ? v[ 1 ] : v[ 0 ] ) = x;
+                ( count ? m[ 1 ] : m[ 0 ] ) = site;
+            }
+            count++;
+        }
+    };
+    __device__ __forceinline__ uint32_t third_site( uint4 r, uint32_t k, uint32_t l )
+    {
+        return ( r.x != k && r.x != l ) ? r.x : ( ( r.y != k && r.y != l ) ? r.y : r.z );
+    }
+
+    // The stored vertices of cell i on its edge (k, l): the ends, the largest radius (at least 0) and
+    // up to two distinct third sites. The records are scanned first and the vertices solved after, so that
+    // the lanes of a warp, whose vertices stand at different places of the store, solve them together.
+    __device__ __forceinline__ double stored_ends( const CellContext & c, uint32_t i, double4 si, uint32_t k, uint32_t l, ArcEnds & ends,
+                                                   uint32_t ( &hint )[ 2 ] )
+    {
+        const uint4 *  store = c.vertices + store_row( c, i ) * kMaxVertices;
+        const uint32_t vn    = c.vertex_nb[ i ];
+        uint32_t       at[ 2 ] = { vn, vn }, more = vn, count = 0;
+        hint[ 0 ] = hint[ 1 ] = kNone;
+        for ( uint32_t v = 0; v < vn; v++ )
+        {
+            const uint4 r = store[ v ];
+            if ( vertex_on_edge( r, k, l ) )
+            {
+                const uint32_t m = third_site( r, k, l );
+                if ( hint[ 0 ] == kNone )
+                    hint[ 0 ] = m;
+                else if ( hint[ 1 ] == kNone && m != hint[ 0 ] )
+                    hint[ 1 ] = m;
+                if ( count == 0 )
+                    at[ 0 ] = v;
+                else if ( count == 1 )
+                    at[ 1 ] = v;
+                else if ( count == 2 )
+                    more = v;
+                count++;
+            }
+        }
+        double wmax = 0.0;
+#pragma unroll 1
+        for ( uint32_t q = 0; q < 2; q++ )
+        {
+            const uint32_t v = q ? at[ 1 ] : at[ 0 ];
+            if ( v < vn )
+            {
+                const uint4   r = store[ v ];
+                const double4 x = solve_vertex( c, si, r );
+                wmax            = fmax( wmax, x.w );
+                ends.add( x, third_site( r, k, l ) );
+            }
+        }
+        for ( uint32_t v = more; v < vn; v++ ) // more than two: rare
+        {
+            const uint4 r = store[ v ];
+            if ( vertex_on_edge( r, k, l ) )
+            {
+                wmax = fmax( wmax, solve_vertex( c, si, r ).w );
+                ends.count++;
+            }
+        }
+        return wmax;
+    }
+
+    // The balls of the arc of trisector (i, k, l) between its two vertices. With c_i as the origin,
+    // e_k = c_k - c_i, d_k = r_k - r_i and rho = w + r_i = |x|, the trisector's points are
+    // x = A + rho B + s n, n the normal of the plane of the centres, A and B in it from
+    // e.x = (|e|^2 - d^2) / 2 - rho d for e_k and e_l; and |x| = rho makes (rho, s) a conic,
+    // s^2 = alpha rho^2 - 2 beta rho - gamma. Whether site j conflicts with the sphere at x is the
+    // sign of |x - e_j|^2 - (rho + d_j)^2, on the conic equal to |e_j|^2 - d_j^2 - 2 (e_j.x + rho d_j):
+    // linear in (rho, s). The arc lies in the triangle of its ends and the meeting point T of their
+    // tangents, so a site that conflicts at none of these three conflicts nowhere on the arc. At
+    // the ends that is a ball each. T lies off the conic by D = |x|^2 - rho^2, and for a sphere of
+    // radius r_j >= 0 the linear form there is at least delta^2 - w^2 - D, delta the distance of
+    // the sphere (or of a box around it) from x: a ball of radius sqrt(w^2 + D). (With equal radii
+    // it passes through the three centres, in the union of the other two: only unequal radii
+    // leave anything to find.) On a hyperbola (of which the points with rho > 0 are one branch) the
+    // arc is the one between the ends; on an ellipse it is the smaller one if on both ends the
+    // third site's conflict fades that way. False where the points do not determine this safely.
+    __device__ __forceinline__ bool arc_reach( const CellContext & c, double4 si, double4 sk, double4 sl, const ArcEnds & ends,
+                                               EdgeReach & reach )
+    {
+        const double3 o   = d3( si );
+        const double3 ek  = d3( sk ) - o, el = d3( sl ) - o;
+        const double  dk  = sk.w - si.w, dl = sl.w - si.w;
+        const double  gkk = ddot( ek, ek ), gll = ddot( el, el ), gkl = ddot( ek, el );
+        const double  det = gkk * gll - gkl * gkl;
+        if ( !( det > 1e-9 * gkk * gll ) )
+            return false; // centres nearly in line
+        const double  inv = 1.0 / det;
+        const double  ak = .5 * ( gkk - dk * dk ), al = .5 * ( gll - dl * dl );
+        const double3 A = ek * ( ( ak * gll - al * gkl ) * inv ) + el * ( ( al * gkk - ak * gkl ) * inv );
+        const double3 B = ek * ( ( dl * gkl - dk * gll ) * inv ) + el * ( ( dk * gkl - dl * gkk ) * inv );
+        const double3 n = dcross( ek, el ) * rsqrt( det );
+        const double  alpha = 1.0 - ddot( B, B ), beta = ddot( A, B ), gamma = ddot( A, A );
+        const double3 u0 = d3( ends.v[ 0 ] ) - o, u1 = d3( ends.v[ 1 ] ) - o;
+        const double  rho0 = sqrt( ddot( u0, u0 ) ), rho1 = sqrt( ddot( u1, u1 ) );
+        const double  s0 = ddot( u0, n ), s1 = ddot( u1, n );
+        // the vertices lie on the curve (they are solved in another order, and may be badly conditioned)
+        const double3 off0 = A + B * rho0 + n * s0 - u0, off1 = A + B * rho1 + n * s1 - u1;
+        if ( !( ddot( off0, off0 ) <= 1e-8 * ( 1.0 + rho0 ) * ( 1.0 + rho0 )
+                && ddot( off1, off1 ) <= 1e-8 * ( 1.0 + rho1 ) * ( 1.0 + rho1 ) && fmax( rho0, rho1 ) < 1e9 ) )
+            return false;
+        const double slack = 1e-3 * ( 1.0 + fabs( s0 ) + fabs( s1 ) );
+        double       sT = s0, rhoT = rho0;
+        if ( alpha > 1e-6 )
+        {
+            // s_a s + (beta - alpha rho_a) rho = -(beta rho_a + gamma) is the tangent at end a
+            const double m0 = beta - alpha * rho0, m1 = beta - alpha * rho1;
+            const double h0 = -( beta * rho0 + gamma ), h1 = -( beta * rho1 + gamma );
+            const double meet = s0 * m1 - s1 * m0;
+            if ( fabs( s0 - s1 ) >= 1e-3 * slack ) // else the ends coincide
+            {
+                sT   = ( h0 * m1 - h1 * m0 ) / meet;
+                rhoT = ( s0 * h1 - s1 * h0 ) / meet;
+            }
+            if ( !( sT >= fmin( s0, s1 ) - slack && sT <= fmax( s0, s1 ) + slack && rhoT >= -1e-3
+                    && rhoT <= 1.001 * fmax( rho0, rho1 ) + 1e-3 ) )
+                return false;
+            reach.kind = kReachArcPlanes;
+        }
+        else if ( alpha < -1e-6 && beta * beta + alpha * gamma > 0.0 )
+        {
+            // (rho, s) = centre + (ar cos, as sin); c0 and c1 the unit vectors of the ends
+            const double disc = beta * beta + alpha * gamma, rc = beta / alpha;
+            const double ar = sqrt( disc ) / -alpha, as = sqrt( disc / -alpha );
+            if ( !( rc + ar < kFarRoot ) )
+                return false;
+            const double2 c0 = make_double2( ( rho0 - rc ) / ar, s0 / as ), c1 = make_double2( ( rho1 - rc ) / ar, s1 / as );
+            const double  cosine = ddot( c0, c1 );
+            if ( !( cosine > -.5 && fabs( ddot( c0, c0 ) - 1.0 ) < 1e-3 && fabs( ddot( c1, c1 ) - 1.0 ) < 1e-3 ) )
+                return false; // more than a third of the ellipse apart
+            for ( int a = 0; a < 2; a++ )
+            {
+                // the linear form of the third site grows from this end towards the other
+                const double4 sm = c.sites[ a ? ends.m[ 1 ] : ends.m[ 0 ] ];
+                const double3 em = d3( sm ) - o;
+                const double2 from = a ? c1 : c0, to = a ? c0 : c1;
+                const double  dr = ar * ( to.x - cosine * from.x ), ds = as * ( to.y - cosine * from.y );
+                const double  fr = ddot( em, B ) + ( sm.w - si.w ), fs = ddot( em, n );
+                if ( !( -( fr * dr + fs * ds ) > 1e-3 * ( fabs( fr * dr ) + fabs( fs * ds ) ) ) )
+                    return false;
+            }
+            rhoT       = rc + ar * ( c0.x + c1.x ) / ( 1.0 + cosine );
+            sT         = as * ( c0.y + c1.y ) / ( 1.0 + cosine );
+            reach.kind = kReachArc;
+        }
+        else
+            return false;
+        const double3 uT = A + B * rhoT + n * sT;
+        const double  wT = rhoT - si.w;
+        reach.ball[ 0 ]  = reach_ball( d3( ends.v[ 0 ] ), rho0 - si.w );
+        reach.ball[ 1 ]  = reach_ball( d3( ends.v[ 1 ] ), rho1 - si.w );
+        reach.ball[ 2 ]  = reach_ball( o + uT, sqrt( wT * wT + fmax( 0.0, ddot( uT, uT ) - rhoT * rhoT ) ) );
+        return true;
+    }
+
+    // Reach of edge (k, l) of cell i: wmax is the largest radius on its arc, `around` the reference's
+    // bounding sphere of the trisector.
+    __device__ __forceinline__ EdgeReach edge_reach( const CellContext & c, double4 si, double4 sk, double4 sl, bool hyperbola,
+                                                     const ArcEnds & ends, double wmax, float4 around )
+    {
+        EdgeReach    reach;
+        const double rmin = c.scene->rmin;
+        // spheres of negative radius reach out of their boxes by less than four radii
+        const float low = fmaxf( 0.f, float( -4.0 * rmin ) );
+        reach.limit     = reach_ball( d3( si ), 2.0 * wmax + si.w );
+        const float margin = 1e-5f * ( around.w + fabsf( around.x ) + fabsf( around.y ) + fabsf( around.z ) );
+        if ( around.w + margin < reach.limit.w )
+            reach.limit = make_float4( around.x, around.y, around.z, around.w + margin );
+        reach.limit.w += float( c.scene->rmax - rmin ) + low;
+        // a root of radius w touches the plane to L^2 / 2w at a distance of L, at most 2.5 times the
+        // limit's radius
+        reach.margin    = 1e-5f * ( reach.limit.w + fabsf( reach.limit.x ) + fabsf( reach.limit.y ) + fabsf( reach.limit.z ) );
+        reach.slab[ 0 ] = reach.slab[ 1 ] = float( 3.2 / kFarRoot ) * reach.limit.w * reach.limit.w + reach.margin;
+        reach.diameter  = 2.f * fmaxf( 0.f, float( rmin ) );
+        reach.below     = hyperbola && rmin >= 0.0;
+        if ( ends.count == 2 && rmin >= 0.0 && arc_reach( c, si, sk, sl, ends, reach )
+             && ( hyperbola || reach.kind == kReachArc ) )
+            return reach;
+        reach.kind      = kReachBall;
+        reach.ball[ 0 ] = reach.ball[ 1 ] = reach.ball[ 2 ] = reach.limit;
+        return reach;
     }
 
     // An apex (trisector root in the plane of the centres) counts unless a neighbour other
@@ -164,11 +464,26 @@ namespace apo2
         return pen > 1e-4 * ( site.w + fabs( apex.w ) ) + 1e-6;
     }
 
-    // Radius of the ball around c_i that holds every possible contributor, with margins.
-    __device__ __forceinline__ float reach_radius( double wmax, double ri, double rmax )
+    // The node every walk inside a ball may start from: from the root down to where both children
+    // meet the ball. The walk would go the same way, one box after another, without meeting a leaf.
+    __device__ __forceinline__ uint32_t node_around( const WideNode * nodes, uint32_t n, float4 ball, uint32_t node = 0 )
     {
-        const double r = 2.0 * wmax * 1.01 + ri + rmax + 1e-3 * ( 1.0 + wmax );
-        return float( r ) * 1.0001f + 1e-3f;
+        while ( true )
+        {
+            Box      lb, rb;
+            uint32_t lc, rc;
+            load_node( nodes, node, lb, rb, lc, rc );
+            const bool l = meets( ball, lb ), r = meets( ball, rb );
+            const uint32_t next = l ? lc : rc;
+            if ( l == r || next >= n - 1 )
+                return node;
+            node = next;
+        }
+    }
+    // Ball holding every site that a sphere of radius up to w touching sphere i can touch.
+    __device__ __forceinline__ float4 touch_ball( const CellContext & c, double4 si, double w )
+    {
+        return reach_ball( d3( si ), 2.002 * w + si.w + fmax( 0.0, -4.0 * c.scene->rmin ) );
     }
     void configure_cell_kernels();
     // bytes of CellContext::walk_scratch: one region per warp the cell kernels launch

@@ -23,7 +23,7 @@ namespace apo2
     constexpr uint32_t kFlagFound     = 1;
     constexpr uint32_t kFlagOverflow  = 2;
 #ifndef APO2_SPEC_LANE_BUDGET
-#define APO2_SPEC_LANE_BUDGET 256
+#define APO2_SPEC_LANE_BUDGET 512
 #endif
 #ifndef APO2_SPEC_SPLIT_AT
 #define APO2_SPEC_SPLIT_AT 192
@@ -31,19 +31,23 @@ namespace apo2
 #ifndef APO2_SPEC_MIN_BLOCKS
 #define APO2_SPEC_MIN_BLOCKS 4
 #endif
-    constexpr uint32_t kLaneBudget    = APO2_SPEC_LANE_BUDGET; // walk steps one lane may take before the search goes to a warp
+    constexpr uint32_t kLaneBudget    = APO2_SPEC_LANE_BUDGET; // nodes one lane may visit before the search goes to a warp
     constexpr uint32_t kHeavyBlock    = 128;
     constexpr uint32_t kHeavyStack    = 3072; // shared node stack per warp of the cooperative walk
     constexpr uint32_t kSplitAt       = APO2_SPEC_SPLIT_AT; // pending subtrees at which a long walk is handed out
     constexpr uint32_t kSplitSlot     = 0x80000000u; // marks a subtree whose search set-up is cached
 #ifndef APO2_SPEC_REFILL_AT
-#define APO2_SPEC_REFILL_AT 24
+#define APO2_SPEC_REFILL_AT 28
 #endif
     // Idle lanes of a speculation warp fetch and set up new edges together, once at least
     // this many are idle (or none is walking): the set-up (bounding sphere, certificate test)
     // is long FP64 code, and run by one or two lanes at a time it held the warp for most
     // of its time.
     constexpr uint32_t kRefillAt = APO2_SPEC_REFILL_AT;
+#ifndef APO2_SPEC_STEPS
+#define APO2_SPEC_STEPS 16
+#endif
+    constexpr uint32_t kSpecSteps = APO2_SPEC_STEPS; // nodes of every walk between two votes
 #ifndef APO2_BISECTOR_REFILL_AT
 #define APO2_BISECTOR_REFILL_AT 24
 #endif
@@ -179,15 +183,16 @@ namespace apo2
         uint32_t t, e, i, k, l;
         double4  si, sk, sl;
         float4   bsph;
-        float4   reach; // ball around c_i holding every possible contributor
+        EdgeReach reach; // where every possible contributor is
         bool     closed;
-        float3   n1, n2, pp1, pp2;
+        TangentPlanes planes;
         bool     hyperbola;
         const uint32_t * nbr;
         uint32_t nbr_count;
         // the third sites of the edge's vertices: the neighbours bounding its arc, which a
         // candidate root outside the arc almost always lies inside (tested first)
         uint32_t hint[ 2 ];
+        uint32_t from; // node the walk starts at
     };
 
     // Bounding volume of edge (k, l) of cell i and the security-radius test
@@ -200,7 +205,7 @@ namespace apo2
         s.hyperbola   = type == 1;
         const bool   ellipse = type == 2;
         const float4 v1 = to_float( ev0 ), v2 = to_float( ev1 );
-        s.n1 = s.n2 = s.pp1 = s.pp2 = make_float3( 0, 0, 0 );
+        s.planes.n1 = s.planes.n2 = s.planes.p1 = s.planes.p2 = make_float3( 0, 0, 0 );
         if ( ellipse )
         {
             const float3 center = ( f3( v1 ) + f3( v2 ) ) * .5f;
@@ -211,39 +216,25 @@ namespace apo2
         {
             double3 nn1, nn2;
             tangent_planes( s.si, s.sk, s.sl, nn1, nn2 );
-            s.n1             = to_float( nn1 );
-            s.n2             = to_float( nn2 );
+            s.planes.n1      = to_float( nn1 );
+            s.planes.n2      = to_float( nn2 );
             const double3 p1 = d3( s.si ) + nn1 * s.si.w;
             const double3 p2 = d3( s.sk ) + nn1 * s.sk.w;
             const double3 p3 = d3( s.sl ) + nn1 * s.sl.w;
             const double3 p4 = d3( s.si ) + nn2 * s.si.w;
             const double3 p5 = d3( s.sk ) + nn2 * s.sk.w;
             s.bsph           = to_float( sphere_from_points( p1, p2, p3, p5 ) );
-            s.pp1            = to_float( p1 );
-            s.pp2            = to_float( p4 );
+            s.planes.p1      = to_float( p1 );
+            s.planes.p2      = to_float( p4 );
         }
         const float4 fsi    = to_float( s.si );
         const bool   inside = lt_eps( flength( f3( fsi ) - f3( s.bsph ) ), known - s.bsph.w );
         if ( inside )
             return false;
 
-        // reach of the search: largest radius over the edge's arc
-        double         wmax = 0.0;
-        const uint32_t vn   = c.vertex_nb[ s.i ];
-        s.hint[ 0 ] = s.hint[ 1 ] = kNone;
-        for ( uint32_t v = 0; v < vn; v++ )
-        {
-            const uint4 r = c.vertices[ store_row( c, s.i ) * kMaxVertices + v ];
-            if ( vertex_on_edge( r, s.k, s.l ) )
-            {
-                wmax             = fmax( wmax, solve_vertex( c, s.si, r ).w );
-                const uint32_t m = ( r.x != s.k && r.x != s.l ) ? r.x : ( ( r.y != s.k && r.y != s.l ) ? r.y : r.z );
-                if ( s.hint[ 0 ] == kNone )
-                    s.hint[ 0 ] = m;
-                else if ( s.hint[ 1 ] == kNone && m != s.hint[ 0 ] )
-                    s.hint[ 1 ] = m;
-            }
-        }
+        // reach of the search: the arc's ends and its largest radius
+        ArcEnds ends;
+        double  wmax = stored_ends( c, s.i, s.si, s.k, s.l, ends, s.hint );
         if ( ellipse || s.closed )
         {
             const double4 apex[ 2 ] = { ev0, ev1 };
@@ -260,22 +251,60 @@ namespace apo2
                     wmax = fmax( wmax, apex[ a ].w );
             }
         }
-        s.reach = make_float4( fsi.x, fsi.y, fsi.z, reach_radius( wmax, s.si.w, c.scene->rmax ) );
+        s.reach = edge_reach( c, s.si, s.sk, s.sl, s.hyperbola, ends, wmax, s.bsph );
+        if ( s.reach.kind == kReachArcPlanes )
+        {
+            bool open1 = true, open2 = true;
+            for ( uint32_t q = 0; q < s.nbr_count && ( open1 || open2 ); q++ )
+            {
+                const uint32_t u = s.nbr[ q ];
+                if ( u == s.k || u == s.l || u >= c.n )
+                    continue;
+                const float4 m = c.sites_f[ u ];
+                open1          = open1 && !far_roots_blocked( s.planes.n1, fsi, m );
+                open2          = open2 && !far_roots_blocked( s.planes.n2, fsi, m );
+            }
+            if ( !open1 )
+                s.reach.slab[ 0 ] = -FLT_MAX;
+            if ( !open2 )
+                s.reach.slab[ 1 ] = -FLT_MAX;
+            if ( !open1 && !open2 )
+                s.reach.kind = kReachArc;
+        }
+        const uint2 around = c.around[ s.i ];
+        s.from             = wmax <= 1.001 * double( c.largest[ s.i ] ) ? ( s.reach.kind == kReachArc ? around.x : around.y ) : 0u;
+        // only neighbours are tested first, and skipped by the walk
+        for ( uint32_t h = 0; h < 2; h++ )
+            if ( s.hint[ h ] != kNone && !in_sorted( s.nbr, s.nbr_count, s.hint[ h ] ) )
+                s.hint[ h ] = kNone;
         return true;
     }
 
-    // The reference's test for entering a child box (algorithm.inl:642-667: the box meets
-    // the bounding sphere and, for a hyperbolic edge, the closest point of the box lies
-    // below both tangent planes), and the reach test (skipping keeps the visit order).
-    __device__ __forceinline__ bool enter_child( const EdgeSearch & s, const Box & b, float d )
+    // The walk is bound by the node steps (two boxes against three balls and two planes, 50 to 90
+    // nodes an edge); the balls of the arc and the planes replaced the ball around c_i, most of whose
+    // leaves went through a quadrisector solve each. First round's launches, 1M log-normal cloud:
+    // k_edge_speculate 245 -> 102 ms, k_edge_heavy_sub 111 -> 11, k_edge_heavy 20 -> 4; 1M-site protein
+    // packing 117 -> 74, 18.5 -> 8.1, 7.8 -> 3.3 ms; 46^3 lattice 6.6 -> 7.6 ms (equal radii: there
+    // the planes let little in before, and the set-up grew).
+    //
+    // May the box hold a contributor? Without an arc, also the reference's own test for entering it
+    // (algorithm.inl:642-667: the box meets the bounding sphere and, for a hyperbolic edge, the
+    // closest point of the box lies below both tangent planes).
+    __device__ __forceinline__ bool enter_child( const EdgeSearch & s, const Box & b, bool leaf )
     {
-        bool enter = d < 0.f;
+        if ( !within( s.reach, s.planes, b ) )
+            return false;
+        if ( leaf && s.reach.kind != kReachBall )
+            return within( s.reach, s.planes, sphere_in( b ) );
+        if ( s.reach.kind != kReachBall )
+            return true;
+        bool enter = b.distance( s.bsph ) < 0.f;
         if ( s.hyperbola && enter )
         {
             const float3 p = b.closest( s.bsph );
-            enter          = fdot( s.n1, p - s.pp1 ) < 0.f && fdot( s.n2, p - s.pp2 ) < 0.f;
+            enter          = fdot( s.planes.n1, p - s.planes.p1 ) < 0.f && fdot( s.planes.n2, p - s.planes.p2 ) < 0.f;
         }
-        return enter && b.distance( s.reach ) < 0.f;
+        return enter;
     }
 
     // Does site j give the edge two vertices, one of them empty of every other neighbour?
@@ -288,10 +317,11 @@ namespace apo2
         const float4  fj = to_float( sj );
         if ( !intersects( fj, s.bsph ) )
             return false;
-        if ( flength( f3( fj ) - f3( s.reach ) ) > s.reach.w )
+        if ( !within( s.reach, s.planes, fj ) )
             return false;
         if ( s.hyperbola
-             && !( double( fdot( s.n1, f3( fj ) - s.pp1 ) ) < -sj.w && double( fdot( s.n2, f3( fj ) - s.pp2 ) ) < -sj.w ) )
+             && !( double( fdot( s.planes.n1, f3( fj ) - s.planes.p1 ) ) < -sj.w
+                   && double( fdot( s.planes.n2, f3( fj ) - s.planes.p2 ) ) < -sj.w ) )
             return false;
         if ( in_sorted( s.nbr, s.nbr_count, j ) )
             return false;
@@ -304,14 +334,11 @@ namespace apo2
         // A root is empty when no neighbour other than k, l conflicts with it: the neighbours
         // bounding the edge's arc go first (a root outside the arc is nearly always inside one of
         // them), then the whole sorted list. The conjunction is the same.
-        bool hint_ok[ 2 ] = { false, false };
-        for ( uint32_t h = 0; h < 2; h++ )
-            hint_ok[ h ] = s.hint[ h ] != kNone && in_sorted( s.nbr, s.nbr_count, s.hint[ h ] );
         for ( uint32_t r = 0; r < 2; r++ )
         {
             bool ok = true;
             for ( uint32_t h = 0; h < 2 && ok; h++ )
-                if ( hint_ok[ h ] )
+                if ( s.hint[ h ] != kNone )
                     ok = !( c.fp32 ? site_conflict<true>( c, s.hint[ h ], x[ r ], untallied )
                                    : site_conflict<false>( c, s.hint[ h ], x[ r ], untallied ) );
             for ( uint32_t q = 0; q < s.nbr_count && ok; q++ )
@@ -325,6 +352,13 @@ namespace apo2
                 return true;
         }
         return false;
+    }
+
+    __device__ __forceinline__ void send_to_exact( const SpecBuffers & b, uint32_t t, uint32_t e )
+    {
+        // the exact path decides, searching this edge again
+        atomicOr( &b.maybe_bits[ size_t( t ) * kMaybeWords + ( e >> 5 ) ], 1u << ( e & 31 ) );
+        atomicOr( &b.cell_flag[ t ], kFlagFound );
     }
 
     __global__ void __launch_bounds__( kSpecBlock, APO2_SPEC_MIN_BLOCKS ) k_edge_speculate( CellContext c, const uint32_t * __restrict__ tasks,
@@ -404,7 +438,7 @@ namespace apo2
                                 {
                                     active = true;
                                     sp     = 0;
-                                    node   = 0;
+                                    node   = s.from;
                                     steps  = 0;
                                 }
                             }
@@ -413,57 +447,70 @@ namespace apo2
                 }
                 continue;
             }
-            if ( !active )
-                continue;
-
-            // one step of the walk: descend to a leaf (or prune), test it, pop
-            if ( ++steps > kLaneBudget )
+            // some nodes of every walk between two votes. A lane that meets sites to be tested (the leaf
+            // children of its node) waits for the others: the test is long FP64 code.
+            uint32_t found[ 2 ] = { kNone, kNone };
+#pragma unroll 1
+            for ( uint32_t turn = 0; turn < kSpecSteps && active && ( found[ 0 ] & found[ 1 ] ) == kNone; turn++ )
             {
-                // a long search: restart it on a whole warp (k_edge_heavy)
-                const uint32_t slot = atomicAdd( b.heavy_count, 1u );
-                if ( slot < b.heavy_cap )
-                    b.heavy[ slot ] = make_uint2( s.t, s.e );
-                else
+                if ( ++steps > kLaneBudget )
                 {
-                    // exact path instead, with a full search of this edge
-                    atomicOr( &b.maybe_bits[ size_t( s.t ) * kMaybeWords + ( s.e >> 5 ) ], 1u << ( s.e & 31 ) );
-                    atomicOr( &b.cell_flag[ s.t ], kFlagFound );
+                    // a long search: restart it on a whole warp (k_edge_heavy)
+                    const uint32_t slot = atomicAdd( b.heavy_count, 1u );
+                    if ( slot < b.heavy_cap )
+                        b.heavy[ slot ] = make_uint2( s.t, s.e );
+                    else
+                        send_to_exact( b, s.t, s.e ); // with a full search of this edge
+                    active = false;
+                    break;
                 }
-                active = false;
-                continue;
-            }
-            while ( node < n - 1 )
-            {
                 Box      lb, rb;
                 uint32_t lc, rc;
                 load_node( c.nodes, node, lb, rb, lc, rc );
-                const float    dL = lb.distance( s.bsph ), dR = rb.distance( s.bsph );
-                const bool     leftClosest = dL < dR;
-                const uint32_t farChild = leftClosest ? rc : lc, closeChild = leftClosest ? lc : rc;
-                const bool     exploreL = enter_child( s, lb, dL ), exploreR = enter_child( s, rb, dR );
-                const bool     exploreFar = leftClosest ? exploreR : exploreL, exploreClose = leftClosest ? exploreL : exploreR;
-                if ( !exploreFar && !exploreClose )
-                    break;
-                node = exploreClose ? closeChild : farChild;
-                if ( exploreClose && exploreFar )
+                uint32_t   next = kNone;
+                const bool eL = enter_child( s, lb, lc >= n - 1 ), eR = enter_child( s, rb, rc >= n - 1 );
+                if ( eL )
                 {
-                    if ( sp < int( kStack ) )
-                        stack[ sp++ ] = farChild;
+                    if ( lc >= n - 1 )
+                        found[ 0 ] = lc - ( n - 1 );
+                    else
+                        next = lc;
+                }
+                if ( eR )
+                {
+                    if ( rc >= n - 1 )
+                        found[ 1 ] = rc - ( n - 1 );
+                    else if ( next == kNone )
+                        next = rc;
+                    else if ( sp < int( kStack ) )
+                        stack[ sp++ ] = rc;
                     else
                         err |= kErrStack;
                 }
+                // the edge's own sites and the neighbours that bound it touch every ball
+#pragma unroll
+                for ( uint32_t q = 0; q < 2; q++ )
+                    if ( found[ q ] == s.i || found[ q ] == s.k || found[ q ] == s.l || found[ q ] == s.hint[ 0 ] || found[ q ] == s.hint[ 1 ] )
+                        found[ q ] = kNone;
+                if ( next != kNone )
+                    node = next;
+                else if ( sp > 0 )
+                    node = stack[ --sp ];
+                else
+                    active = false; // once the sites found are tested
             }
-            if ( node >= n - 1 && node < 2 * n - 1 && contributes( c, s, node - ( n - 1 ) ) )
+            // the sites found, of all lanes together
+#pragma unroll 1
+            for ( uint32_t q = 0; q < 2; q++ )
             {
-                atomicOr( &b.maybe_bits[ size_t( s.t ) * kMaybeWords + ( s.e >> 5 ) ], 1u << ( s.e & 31 ) );
-                atomicOr( &b.cell_flag[ s.t ], kFlagFound );
-                active = false;
-                continue;
+                const uint32_t j = q ? found[ 1 ] : found[ 0 ];
+                if ( j != kNone && contributes( c, s, j ) )
+                {
+                    send_to_exact( b, s.t, s.e );
+                    active = false;
+                    break;
+                }
             }
-            if ( sp == 0 )
-                active = false;
-            else
-                node = stack[ --sp ];
         }
         if ( err )
             atomicOr( error, err );
@@ -507,8 +554,8 @@ namespace apo2
                 {
                     Box lb, rb;
                     load_node( c.nodes, node, lb, rb, lc, rc );
-                    eL = enter_child( s, lb, lb.distance( s.bsph ) );
-                    eR = enter_child( s, rb, rb.distance( s.bsph ) );
+                    eL = enter_child( s, lb, lc >= n - 1 );
+                    eR = enter_child( s, rb, rc >= n - 1 );
                 }
             }
             if ( __any_sync( 0xffffffffu, hit ) )
@@ -554,13 +601,6 @@ namespace apo2
         setup_edge( c, s, c.known_radii[ s.i ] ); // the lane path already found it needs a search
     }
 
-    __device__ __forceinline__ void send_to_exact( const SpecBuffers & b, uint32_t t, uint32_t e )
-    {
-        // the exact path decides, searching this edge again
-        atomicOr( &b.maybe_bits[ size_t( t ) * kMaybeWords + ( e >> 5 ) ], 1u << ( e & 31 ) );
-        atomicOr( &b.cell_flag[ t ], kFlagFound );
-    }
-
     __global__ void __launch_bounds__( kHeavyBlock, 4 ) k_edge_heavy( CellContext c, const uint32_t * __restrict__ tasks,
                                                                       SpecBuffers b, uint32_t * error )
     {
@@ -589,7 +629,7 @@ namespace apo2
             search_of_heavy( c, tasks, b, h, s );
             uint32_t size = 1;
             if ( lane == 0 )
-                st[ 0 ] = 0;
+                st[ 0 ] = s.from;
             __syncwarp();
             const uint32_t end = cooperative_walk( c, s, st, size, kSplitAt );
             if ( end == kWalkSplit )
