@@ -2542,6 +2542,8 @@ namespace apo2
         return std::max( 1, std::min( cell_grid_slot(), needed ) );
     }
 
+    int cell_grid_blocks( uint32_t cells ) { return cell_grid( cells ); }
+
     void launch_knn( const CellContext & c, uint32_t step, cudaStream_t s )
     {
         const uint32_t blocks = ( c.n + kKnnBlock - 1 ) / kKnnBlock;

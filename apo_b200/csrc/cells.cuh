@@ -132,6 +132,18 @@ namespace apo2
     constexpr uint32_t kCoopWidth        = APO2_COOP_WIDTH; // frontier nodes per lane per step
     constexpr uint32_t kCoopCap          = 8192;
     constexpr uint32_t kWalkScratchWords = kCoopCap + 32 * ( kStack + 1 );
+    // The edge search keeps a cell's surroundings in the same scratch: up to kListCap sites
+    // (float4, then ids) and the stack of the walk that collects them. An edge's walk is 50 to 90
+    // nodes whatever the density, its share of the list grows with it. Edge search of all kernels, with
+    // lists of up to 64 / 128 / 256 / 384 / 1024 sites (0: 75.5, 105.9 and 7.7 ms): 1M protein packing
+    // 76.9 / 73.8 / 72.7 / 74.6 / 88.6 ms, 1M log-normal cloud 112 / 107 / 86 / 83 / 75 ms, 46^3
+    // lattice 6.0 / 5.9 / 6.0 / 5.8 / 5.9 ms.
+#ifndef APO2_EDGE_LIST
+#define APO2_EDGE_LIST 384
+#endif
+    constexpr uint32_t kListCap   = APO2_EDGE_LIST;
+    constexpr uint32_t kListStack = 4096;
+    static_assert( 5 * kListCap + kListStack <= kWalkScratchWords && kWalkScratchWords % 4 == 0, "the list fits the scratch" );
 
     // Position of a stored vertex: root `type` of quadrisector(si, sj, sk, sl) with the
     // sorted ids (topology_update.inl:104-111).
@@ -485,7 +497,68 @@ namespace apo2
     {
         return reach_ball( d3( si ), 2.002 * w + si.w + fmax( 0.0, -4.0 * c.scene->rmin ) );
     }
+    // The sites that reach into the ball, other than i, the buried ones and those that `skip` names,
+    // collected by the warp from `node` down. Returns their number, or kNone if there are more than
+    // kListCap.
+    template<class Skip>
+    __device__ __forceinline__ uint32_t collect_sites( const CellContext & c, uint32_t i, float4 ball, uint32_t node, float4 * sites,
+                                                       uint32_t * ids, uint32_t * stack, Skip && skip )
+    {
+        constexpr uint32_t all   = 0xffffffffu;
+        const uint32_t     lane  = threadIdx.x & 31, n = c.n;
+        const uint32_t below = ( 1u << lane ) - 1u;
+        uint32_t       size = 1, found = 0;
+        if ( lane == 0 )
+            stack[ 0 ] = node;
+        __syncwarp();
+        while ( size > 0 )
+        {
+            const uint32_t take = min( size, 32u );
+            size -= take;
+            uint32_t child[ 2 ] = { 0, 0 };
+            bool     in[ 2 ]    = { false, false };
+            if ( lane < take )
+            {
+                Box lb, rb;
+                load_node( c.nodes, stack[ size + lane ], lb, rb, child[ 0 ], child[ 1 ] );
+                in[ 0 ] = meets( ball, lb );
+                in[ 1 ] = meets( ball, rb );
+            }
+            __syncwarp();
+#pragma unroll 1
+            for ( uint32_t q = 0; q < 2; q++ )
+            {
+                const uint32_t x    = q ? child[ 1 ] : child[ 0 ];
+                const bool     here = q ? in[ 1 ] : in[ 0 ];
+                const uint32_t j    = x - ( n - 1 );
+                bool           site = here && x >= n - 1 && j != i;
+                float4         s    = make_float4( 0, 0, 0, 0 );
+                if ( site )
+                {
+                    s    = c.sites_f[ j ];
+                    site = meets( ball, s ) && c.status[ j ] != kBuried && !skip( j );
+                }
+                const uint32_t leaves = __ballot_sync( all, site ), nodes = __ballot_sync( all, here && x < n - 1 );
+                if ( found + __popc( leaves ) > kListCap || size + __popc( nodes ) > kListStack )
+                    return kNone;
+                if ( site )
+                {
+                    sites[ found + __popc( leaves & below ) ] = s;
+                    ids[ found + __popc( leaves & below ) ]   = j;
+                }
+                if ( here && x < n - 1 )
+                    stack[ size + __popc( nodes & below ) ] = x;
+                found += __popc( leaves );
+                size += __popc( nodes );
+            }
+            __syncwarp();
+        }
+        return found;
+    }
+
     void configure_cell_kernels();
+    // blocks of kCellBlock threads that the cell kernels are launched with, one walk-scratch region per warp
+    int cell_grid_blocks( uint32_t cells );
     // bytes of CellContext::walk_scratch: one region per warp the cell kernels launch
     size_t walk_scratch_bytes();
     // k_cells modes: first kNN step, a later kNN step, initial cells only (no kNN step)

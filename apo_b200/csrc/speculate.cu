@@ -23,7 +23,7 @@ namespace apo2
     constexpr uint32_t kFlagFound     = 1;
     constexpr uint32_t kFlagOverflow  = 2;
 #ifndef APO2_SPEC_LANE_BUDGET
-#define APO2_SPEC_LANE_BUDGET 512
+#define APO2_SPEC_LANE_BUDGET 160
 #endif
 #ifndef APO2_SPEC_SPLIT_AT
 #define APO2_SPEC_SPLIT_AT 192
@@ -31,7 +31,10 @@ namespace apo2
 #ifndef APO2_SPEC_MIN_BLOCKS
 #define APO2_SPEC_MIN_BLOCKS 4
 #endif
-    constexpr uint32_t kLaneBudget    = APO2_SPEC_LANE_BUDGET; // nodes one lane may visit before the search goes to a warp
+    // Nodes one lane may visit before the search goes to a warp. The lane kernel lasts as long as its
+    // longest walk, some 1.9 us a node: of 128 / 256 / 512 nodes, 10k uniform sites 5.8 / 6.2 / 6.5 ms,
+    // 1M log-normal cloud 321 / 318 / 318 ms.
+    constexpr uint32_t kLaneBudget    = APO2_SPEC_LANE_BUDGET;
     constexpr uint32_t kHeavyBlock    = 128;
     constexpr uint32_t kHeavyStack    = 3072; // shared node stack per warp of the cooperative walk
     constexpr uint32_t kSplitAt       = APO2_SPEC_SPLIT_AT; // pending subtrees at which a long walk is handed out
@@ -193,6 +196,7 @@ namespace apo2
         // candidate root outside the arc almost always lies inside (tested first)
         uint32_t hint[ 2 ];
         uint32_t from; // node the walk starts at
+        bool     covered; // the reach lies in what the cell's vertex spheres can touch
     };
 
     // Bounding volume of edge (k, l) of cell i and the security-radius test
@@ -272,7 +276,8 @@ namespace apo2
                 s.reach.kind = kReachArc;
         }
         const uint2 around = c.around[ s.i ];
-        s.from             = wmax <= 1.001 * double( c.largest[ s.i ] ) ? ( s.reach.kind == kReachArc ? around.x : around.y ) : 0u;
+        s.covered          = wmax <= 1.001 * double( c.largest[ s.i ] );
+        s.from             = s.covered ? ( s.reach.kind == kReachArc ? around.x : around.y ) : 0u;
         // only neighbours are tested first, and skipped by the walk
         for ( uint32_t h = 0; h < 2; h++ )
             if ( s.hint[ h ] != kNone && !in_sorted( s.nbr, s.nbr_count, s.hint[ h ] ) )
@@ -361,6 +366,100 @@ namespace apo2
         atomicOr( &b.cell_flag[ t ], kFlagFound );
     }
 
+    // Edge e of task t, ready for the search; false if it needs none.
+    __device__ __forceinline__ bool load_edge( const CellContext & c, const uint32_t * tasks, const SpecBuffers & b, uint32_t t,
+                                               uint32_t e, EdgeSearch & s )
+    {
+        s.t           = t;
+        s.e           = e;
+        s.i           = tasks[ t ];
+        const uint4 r = c.edges[ store_row( c, s.i ) * kMaxEdges + e ];
+        s.k           = r.x;
+        s.l           = r.y;
+        s.closed      = r.z == kNone;
+        s.si          = c.sites[ s.i ];
+        s.nbr         = b.nbr + size_t( t ) * kNbrCap;
+        s.nbr_count   = b.nbr_count[ t ];
+        // an edge validated before is not searched (algorithm.inl:522-526, 552)
+        if ( ( r.w & 0xffu ) == 1u )
+            return false;
+        s.sk = c.sites[ s.k ];
+        s.sl = c.sites[ s.l ];
+        return setup_edge( c, s, c.known_radii[ s.i ] );
+    }
+
+    // Edges of cells with few surroundings, nearly all: a warp per cell collects the sites, other than
+    // the neighbours, within the bound of the cell's edges (some hundred), and its lanes, an edge
+    // each, go through that list together. Per edge that is some hundred tests of a sphere against
+    // three balls, read by all lanes at once, where a walk of its own took 50 to 90 nodes of two boxes
+    // each, on lanes that part at every node. Cells with more surroundings than the list holds (hull
+    // cells) keep their items for k_edge_speculate, edges that reach past the list go to a warp of
+    // their own (k_edge_heavy). All edge-search kernels of a build: 1M log-normal cloud 124 -> 103 ms,
+    // 46^3 lattice 8.2 -> 6.2 ms, 100k uniform 14.0 -> 9 ms, 10k uniform 1.9 -> 1.8 ms, 1M-site protein
+    // packing 87 -> 86 ms.
+    __global__ void __launch_bounds__( kCellBlock, 4 ) k_edge_cells( CellContext c, const uint32_t * __restrict__ tasks,
+                                                                     const uint32_t * __restrict__ task_count, SpecBuffers b )
+    {
+        const uint32_t warp  = threadIdx.x >> 5, lane = lane_of();
+        const uint32_t gwarp = blockIdx.x * ( kCellBlock / 32 ) + warp;
+        const uint32_t count = *task_count;
+        float4 *       list  = reinterpret_cast<float4 *>( c.walk_scratch + size_t( gwarp ) * kWalkScratchWords );
+        uint32_t *     ids   = reinterpret_cast<uint32_t *>( list + kListCap );
+        const Scene &  scene = *c.scene;
+        const float    density = float( c.n ) / float( ( scene.hi[ 0 ] - scene.lo[ 0 ] ) * ( scene.hi[ 1 ] - scene.lo[ 1 ] ) * ( scene.hi[ 2 ] - scene.lo[ 2 ] ) );
+        while ( true )
+        {
+            uint32_t t = 0;
+            if ( lane == 0 )
+                t = atomicAdd( c.work_counter, 1u );
+            t = __shfl_sync( 0xffffffffu, t, 0 );
+            if ( t >= count )
+                break;
+            const uint32_t i = tasks[ t ], edges = b.item_count[ t ]; // none where the cell needs no search
+            if ( edges == 0 )
+                continue;
+            const uint32_t * nbr   = b.nbr + size_t( t ) * kNbrCap;
+            const uint32_t   known = b.nbr_count[ t ];
+            float4           ball  = touch_ball( c, c.sites[ i ], c.largest[ i ] );
+            ball.w += 1.001f * float( c.scene->rmax - c.scene->rmin );
+            // far more than the list holds, at the scene's mean density: not worth collecting
+            if ( 4.2f * ball.w * ball.w * ball.w * density > 4.f * float( kListCap ) )
+                continue;
+            const uint32_t listed = collect_sites( c, i, ball, c.around[ i ].y, list, ids, ids + kListCap,
+                                                   [ & ]( uint32_t j ) { return in_sorted( nbr, known, j ); } );
+            if ( listed == kNone )
+                continue; // its items stay
+            for ( uint32_t base = 0; base < edges; base += 32 )
+            {
+                EdgeSearch s;
+                bool       open = base + lane < edges && load_edge( c, tasks, b, t, base + lane, s );
+                if ( open && !s.covered )
+                {
+                    const uint32_t slot = atomicAdd( b.heavy_count, 1u );
+                    if ( slot < b.heavy_cap )
+                        b.heavy[ slot ] = make_uint2( s.t, s.e );
+                    else
+                        send_to_exact( b, s.t, s.e );
+                    open = false;
+                }
+                for ( uint32_t q = 0; q < listed; q++ )
+                {
+                    const bool near = open && within( s.reach, s.planes, list[ q ] );
+                    if ( !__any_sync( 0xffffffffu, near ) )
+                        continue;
+                    if ( near && contributes( c, s, ids[ q ] ) )
+                    {
+                        send_to_exact( b, s.t, s.e );
+                        open = false;
+                    }
+                }
+            }
+            if ( lane == 0 )
+                b.item_count[ t ] = 0;
+            __syncwarp();
+        }
+    }
+
     __global__ void __launch_bounds__( kSpecBlock, APO2_SPEC_MIN_BLOCKS ) k_edge_speculate( CellContext c, const uint32_t * __restrict__ tasks,
                                                                       const uint32_t * __restrict__ task_count,
                                                                       SpecBuffers b, uint32_t * error )
@@ -419,29 +518,12 @@ namespace apo2
                             // no neighbour list for this cell: the exact path searches this edge
                             atomicOr( &b.maybe_bits[ size_t( s.t ) * kMaybeWords + ( e >> 5 ) ], 1u << ( e & 31 ) );
                         }
-                        else
+                        else if ( load_edge( c, tasks, b, lo, e, s ) )
                         {
-                            s.i           = tasks[ s.t ];
-                            const uint4 r = c.edges[ store_row( c, s.i ) * kMaxEdges + e ];
-                            s.k           = r.x;
-                            s.l           = r.y;
-                            s.closed      = r.z == kNone;
-                            s.si          = c.sites[ s.i ];
-                            s.nbr         = b.nbr + size_t( s.t ) * kNbrCap;
-                            s.nbr_count   = b.nbr_count[ s.t ];
-                            // an edge validated before is not searched (algorithm.inl:522-526, 552)
-                            if ( ( r.w & 0xffu ) != 1u )
-                            {
-                                s.sk = c.sites[ s.k ];
-                                s.sl = c.sites[ s.l ];
-                                if ( setup_edge( c, s, c.known_radii[ s.i ] ) )
-                                {
-                                    active = true;
-                                    sp     = 0;
-                                    node   = s.from;
-                                    steps  = 0;
-                                }
-                            }
+                            active = true;
+                            sp     = 0;
+                            node   = s.from;
+                            steps  = 0;
                         }
                     }
                 }
@@ -1059,10 +1141,12 @@ namespace apo2
         const int heavy_grid = dev >= 0 ? g_heavy_grid[ dev ] : 148 * 4;
         const uint32_t nbr_blocks = std::max( 1u, std::min<uint32_t>( ( c.n + 3 ) / 4, 148 * 32 ) );
         APO2_LAUNCH( "k_neighbor_lists", s, k_neighbor_lists<false><<<nbr_blocks, kNbrBlock, 0, s>>>( c, tasks, task_count, b ) );
+        cudaMemsetAsync( b.heavy_count, 0, sizeof( uint32_t ), s );
+        cudaMemsetAsync( c.work_counter, 0, sizeof( uint32_t ), s );
+        APO2_LAUNCH( "k_edge_cells", s, k_edge_cells<<<cell_grid_blocks( c.n ), kCellBlock, 0, s>>>( c, tasks, task_count, b ) );
         scan_exclusive( b.item_count, c.n, b.scan_sums, b.item_total, s );
         cudaMemsetAsync( b.item_counter, 0, sizeof( uint64_t ), s );
         cudaMemsetAsync( b.exact_count, 0, sizeof( uint32_t ), s );
-        cudaMemsetAsync( b.heavy_count, 0, sizeof( uint32_t ), s );
         cudaMemsetAsync( b.heavy_next, 0, sizeof( uint32_t ), s );
         cudaMemsetAsync( b.sub_count, 0, sizeof( uint32_t ), s );
         cudaMemsetAsync( b.sub_next, 0, sizeof( uint32_t ), s );
