@@ -471,6 +471,8 @@ namespace
         spec_carve( h->spec, a.take<char>( spec_bytes( n ) ), n );
         c.walk_scratch    = a.take<uint32_t>( walk_scratch_bytes() / sizeof( uint32_t ) );
         c.work_counter    = a.take<uint32_t>( 1 );
+        c.deferred        = h->spec.exact_tasks; // not in use while the cell passes run
+        c.deferred_count  = h->spec.exact_count;
         c.counters        = a.take<unsigned long long>( kCounters );
         c.largest         = a.take<float>( n );
         c.around          = a.take<uint2>( n );

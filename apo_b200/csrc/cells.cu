@@ -20,6 +20,7 @@ namespace apo2
 {
     constexpr uint32_t kFull        = 0xffffffffu;
     constexpr uint32_t kMaxRestarts = 4096; // bound of the restart loops of the edge / bisector passes
+    constexpr uint32_t kErrDefer    = 1u << 31; // small slots: a record was dropped, the cell is done again
 
     __device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31; }
     __device__ __forceinline__ uint32_t highest( uint32_t m ) { return 31u - __clz( m ); }
@@ -56,15 +57,16 @@ namespace apo2
     // The cell of one warp, in shared memory
     // -----------------------------------------------------------------------------------
     // Fp32: the filtered form's instantiation (apo2_options.precision).
-    template<bool Fp32>
-    struct WarpCell
+    template<bool Fp32, bool Small = false>
+    struct WarpCell : CellSlots<Small>
     {
-        uint4 * v;       // (j, k, l, type | status << 8), capacity kVertexSlots
+        static constexpr bool kFp32 = Fp32, kSmall = Small;
+        uint4 * v;       // (j, k, l, type | status << 8), capacity kVertices
         double4 * pos;   // solved position of v[*]
-        uint4 * e;       // (j, k, vertex count, status | validated << 8), capacity kEdgeSlots
-        uint32_t * u;    // distinct sites of e[*] (the cell's neighbours), capacity kSiteSlots
+        uint4 * e;       // (j, k, vertex count, status | validated << 8), capacity kEdges
+        uint32_t * u;    // distinct sites of e[*] (the cell's neighbours), capacity kSites
         uint32_t vn, en; // warp-uniform sizes
-        uint32_t un;     // neighbours in u, or kNone: more than kSiteSlots, e[*] is scanned instead
+        uint32_t un;     // neighbours in u, or kNone: more than kSites, e[*] is scanned instead
         mutable FilterTally tally; // this lane's FP32-filter counts
     };
 
@@ -112,7 +114,7 @@ namespace apo2
                 for ( uint32_t q = 0; q < n; q++ )
                     add = add && w.u[ q ] != id;
                 const uint32_t bal = __ballot_sync( kFull, add );
-                if ( n + __popc( bal ) > kSiteSlots )
+                if ( n + __popc( bal ) > W::kSites )
                 {
                     w.un = kNone;
                     return;
@@ -132,7 +134,7 @@ namespace apo2
     __device__ __forceinline__ void relist_sites( W & w, uint32_t j )
     {
         const uint32_t lane = lane_id();
-        if ( w.un >= kSiteSlots ) // no list, or none to spare for j
+        if ( w.un >= W::kSites ) // no list, or none to spare for j
         {
             list_sites( w );
             return;
@@ -164,8 +166,8 @@ namespace apo2
     // of the cell's edges other than skip1 / skip2 intersects `sphere`. Warp-collective, one sphere;
     // returns the warp-wide result. The loop stops once a conflict is known, which does not
     // change the result.
-    template<bool Fp32>
-    __device__ __forceinline__ bool edges_clear( const CellContext & c, const WarpCell<Fp32> & w, double4 sphere, uint32_t skip1,
+    template<class W>
+    __device__ __forceinline__ bool edges_clear( const CellContext & c, const W & w, double4 sphere, uint32_t skip1,
                                                  uint32_t skip2 )
     {
         bool               ok    = true;
@@ -178,7 +180,7 @@ namespace apo2
             {
                 const uint32_t id = sites[ q ];
                 if ( id != skip1 && id != skip2 )
-                    ok = !site_conflict<Fp32>( c, id, sphere, w.tally );
+                    ok = !site_conflict<W::kFp32>( c, id, sphere, w.tally );
             }
             if ( !__all_sync( kFull, ok ) )
                 return false;
@@ -192,8 +194,8 @@ namespace apo2
     // one lane's sphere at a time with a neighbour per lane, as the reference does, spent 65 to
     // 80 % of the update on votes and shuffles around few tests: cells have 8 to 13 neighbours
     // while 20 to 50 spheres are checked per update.)
-    template<bool Fp32>
-    __device__ __forceinline__ uint32_t spheres_clear( const CellContext & c, const WarpCell<Fp32> & w, double4 x0, double4 x1,
+    template<class W>
+    __device__ __forceinline__ uint32_t spheres_clear( const CellContext & c, const W & w, double4 x0, double4 x1,
                                                        uint32_t open, uint32_t skip1, uint32_t skip2 )
     {
         const SiteSequence sites = sites_of( w );
@@ -205,9 +207,9 @@ namespace apo2
             const uint32_t id = sites[ q ];
             if ( id != skip1 && id != skip2 )
             {
-                if ( ( open & 1u ) && site_conflict<Fp32>( c, id, x0, w.tally ) )
+                if ( ( open & 1u ) && site_conflict<W::kFp32>( c, id, x0, w.tally ) )
                     open &= ~1u;
-                if ( ( open & 2u ) && site_conflict<Fp32>( c, id, x1, w.tally ) )
+                if ( ( open & 2u ) && site_conflict<W::kFp32>( c, id, x1, w.tally ) )
                     open &= ~2u;
             }
         }
@@ -224,15 +226,15 @@ namespace apo2
                 return true;
         return false;
     }
-    template<bool Fp32>
-    __device__ __forceinline__ bool clear_by_lane( const CellContext & c, const WarpCell<Fp32> & w, double4 sphere, uint32_t skip1,
+    template<class W>
+    __device__ __forceinline__ bool clear_by_lane( const CellContext & c, const W & w, double4 sphere, uint32_t skip1,
                                                    uint32_t skip2 )
     {
         const SiteSequence sites = sites_of( w );
         for ( uint32_t q = 0; q < sites.count; q++ )
         {
             const uint32_t id = sites[ q ];
-            if ( id != skip1 && id != skip2 && site_conflict<Fp32>( c, id, sphere, w.tally ) )
+            if ( id != skip1 && id != skip2 && site_conflict<W::kFp32>( c, id, sphere, w.tally ) )
                 return false;
         }
         return true;
@@ -337,11 +339,11 @@ namespace apo2
             if ( first )
             {
                 const uint32_t dst = w.en + rank;
-                if ( dst < kEdgeSlots )
+                if ( dst < W::kEdges )
                     w.e[ dst ] = make_uint4( min( j, key ), max( j, key ),
                                              ( peers & closed ) && !( peers & two ) ? kNone : __popc( peers ), 0u );
                 else
-                    err |= kErrEdgeCap;
+                    err |= W::kSmall ? kErrDefer : uint32_t( kErrEdgeCap );
             }
             return written;
         }
@@ -372,10 +374,10 @@ namespace apo2
             {
                 const uint32_t other = v >> 2;
                 const uint32_t dst   = w.en + woff;
-                if ( dst < kEdgeSlots )
+                if ( dst < W::kEdges )
                     w.e[ dst ] = make_uint4( min( j, other ), max( j, other ), ( v & 1u ) ? kNone : uint32_t( f - before ), 0u );
                 else
-                    err |= kErrEdgeCap;
+                    err |= W::kSmall ? kErrDefer : uint32_t( kErrEdgeCap );
                 woff++;
                 before = f;
             }
@@ -405,8 +407,8 @@ namespace apo2
     // kNN cells from 129 to 71 ms and its vertex validation from 265 to 189 ms, the 1M log-normal
     // cloud's from 115 to 61 and from 140 to 106 ms; waits for instructions are 1.7 of 9.2 cycles.
     // -----------------------------------------------------------------------------------
-    template<bool Fp32>
-    __device__ bool update_cell( const CellContext & c, WarpCell<Fp32> & w, uint32_t i, double4 si, uint32_t j, double4 sj,
+    template<class W>
+    __device__ bool update_cell( const CellContext & c, W & w, uint32_t i, double4 si, uint32_t j, double4 sj,
                                  uint32_t & err )
     {
         const uint32_t lane = lane_id();
@@ -445,7 +447,7 @@ namespace apo2
             bool           invalid = false;
             if ( id < baseV )
             {
-                invalid = sphere_conflict<Fp32>( sj, w.pos[ id ], w.tally );
+                invalid = sphere_conflict<W::kFp32>( sj, w.pos[ id ], w.tally );
                 if ( invalid )
                     w.v[ id ].w |= 0xff00u;
             }
@@ -478,7 +480,7 @@ namespace apo2
         for ( uint32_t es = 0; es <= baseE / 32; es++ )
         {
             const uint32_t e   = lane + 32 * es;
-            const uint4    r   = e < kEdgeSlots ? w.e[ e ] : make_uint4( 0, 0, 0, 0 );
+            const uint4    r   = e < W::kEdges ? w.e[ e ] : make_uint4( 0, 0, 0, 0 );
             bool           has = e < baseE;
             const uint32_t k = r.x, l = r.y;
             uint32_t       mask = 0;
@@ -552,13 +554,13 @@ namespace apo2
                 {
                     if ( !( ( valid >> nv ) & 1u ) )
                         continue;
-                    if ( dst < kVertexSlots )
+                    if ( dst < W::kVertices )
                     {
                         w.v[ dst ]   = make_uint4( jj, kk, ll, nv );
                         w.pos[ dst ] = nv ? q1 : q0;
                     }
                     else
-                        err |= kErrVertexCap;
+                        err |= W::kSmall ? kErrDefer : uint32_t( kErrVertexCap );
                     dst++;
                 }
             }
@@ -595,7 +597,7 @@ namespace apo2
                 if ( !__any_sync( kFull, can ) )
                     continue;
                 const uint32_t e = lane + 32 * es;
-                const uint4    r = e < kEdgeSlots ? w.e[ e ] : make_uint4( 0, 0, 0, 0 );
+                const uint4    r = e < W::kEdges ? w.e[ e ] : make_uint4( 0, 0, 0, 0 );
 #pragma unroll 1
                 for ( uint32_t s = 0; s < 2; s++ )
                 {
@@ -629,8 +631,8 @@ namespace apo2
         const uint32_t written = append_edges( w, ne, j, err );
         w.en += written;
         check_capacity( w, err );
-        w.vn = min( w.vn, kVertexSlots );
-        w.en = min( w.en, kEdgeSlots );
+        w.vn = min( w.vn, W::kVertices );
+        w.en = min( w.en, W::kEdges );
         __syncwarp();
 
         // 5. Stable compaction of the marked vertices and the emptied edges (:520-542); without
@@ -734,20 +736,39 @@ namespace apo2
     // -----------------------------------------------------------------------------------
     // Shared-memory carving and the per-cell store
     // -----------------------------------------------------------------------------------
-    template<bool Fp32>
-    __device__ __forceinline__ WarpCell<Fp32> carve( unsigned char * smem, uint32_t warp, uint32_t extra )
+    template<class W>
+    __device__ __forceinline__ W carve( unsigned char * smem, uint32_t warp, uint32_t extra )
     {
-        unsigned char * base = smem + size_t( warp ) * ( kWarpCellBytes + extra );
-        WarpCell<Fp32>  w;
+        unsigned char * base = smem + size_t( warp ) * ( W::kBytes + extra );
+        W               w;
         w.pos = reinterpret_cast<double4 *>( base );
-        w.v   = reinterpret_cast<uint4 *>( base + sizeof( double4 ) * kVertexSlots );
-        w.e   = reinterpret_cast<uint4 *>( base + ( sizeof( double4 ) + sizeof( uint4 ) ) * kVertexSlots );
-        w.u   = reinterpret_cast<uint32_t *>( w.e + kEdgeSlots );
+        w.v   = reinterpret_cast<uint4 *>( base + sizeof( double4 ) * W::kVertices );
+        w.e   = reinterpret_cast<uint4 *>( base + ( sizeof( double4 ) + sizeof( uint4 ) ) * W::kVertices );
+        w.u   = reinterpret_cast<uint32_t *>( w.e + W::kEdges );
         w.vn    = 0;
         w.en    = 0;
         w.un    = 0;
         w.tally = FilterTally {};
         return w;
+    }
+
+    // Small slots: has the cell outgrown them (warp-wide)? The caller then leaves it, with the error
+    // flags it had before, to the launch over the deferred cells.
+    template<class W>
+    __device__ __forceinline__ bool outgrown( uint32_t err )
+    {
+        return W::kSmall && __any_sync( kFull, err & kErrDefer );
+    }
+    template<class W>
+    __device__ __forceinline__ bool too_large( const CellContext & c, uint32_t i )
+    {
+        return W::kSmall && ( c.vertex_nb[ i ] > W::kVertices || c.edge_nb[ i ] > W::kEdges );
+    }
+    __device__ __forceinline__ void defer_cell( const CellContext & c, uint32_t i )
+    {
+        if ( lane_id() == 0 )
+            c.deferred[ atomicAdd( c.deferred_count, 1u ) ] = i;
+        __syncwarp();
     }
 
     template<class W>
@@ -801,11 +822,11 @@ namespace apo2
             atomicOr( c.error, err );
     }
     // Error flags and the FP32 filter's counts of a warp at the end of a kernel.
-    template<bool Fp32>
-    __device__ __forceinline__ void report( const CellContext & c, uint32_t err, const WarpCell<Fp32> & w )
+    template<class W>
+    __device__ __forceinline__ void report( const CellContext & c, uint32_t err, const W & w )
     {
         report( c, err );
-        if ( Fp32 && c.counters )
+        if ( W::kFp32 && c.counters )
         {
             const uint32_t tests = __reduce_add_sync( kFull, w.tally.tests );
             const uint32_t esc   = __reduce_add_sync( kFull, w.tally.escalated );
@@ -1036,14 +1057,16 @@ namespace apo2
     // initializeDataStructure, topology_update.inl:5-47, fused in); kCellsNext continues the
     // stored cells with the next kNN step; kCellsInitOnly writes the initial cells, statuses
     // and known radii alone (no kNN step at all).
-    template<bool Fp32>
-    __global__ void __launch_bounds__( kCellBlock, 4 ) k_cells( CellContext c, uint32_t mode )
+    // Over all cells, or with `deferred` over those that the launch before it, with small slots, left.
+    template<bool Fp32, bool Small>
+    __global__ void __launch_bounds__( kCellBlock, 4 ) k_cells( CellContext c, uint32_t mode, bool deferred )
     {
         extern __shared__ __align__( 16 ) unsigned char smem[];
         const uint32_t warp  = threadIdx.x >> 5;
         const uint32_t gwarp = blockIdx.x * ( kCellBlock / 32 ) + warp;
         const uint32_t nwarp = gridDim.x * ( kCellBlock / 32 );
-        WarpCell<Fp32> w = carve<Fp32>( smem, warp, 0 );
+        using W = WarpCell<Fp32, Small>;
+        W              w = carve<W>( smem, warp, 0 );
         uint32_t       err   = 0;
         // per-warp counters (lane 0 counts), added to the build's counters at the end
         __shared__ uint32_t s_counts[ kCellBlock / 32 ][ kCounters ];
@@ -1054,14 +1077,16 @@ namespace apo2
         // cells are taken one at a time from a shared counter (uneven cells, see bisector pass)
         ( void ) gwarp;
         ( void ) nwarp;
+        const uint32_t total = deferred ? *c.deferred_count : c.hi - c.lo;
         while ( true )
         {
-            uint32_t i = 0;
+            uint32_t t = 0;
             if ( lane_id() == 0 )
-                i = c.lo + atomicAdd( c.work_counter, 1u );
-            i = __shfl_sync( kFull, i, 0 );
-            if ( i >= c.hi )
+                t = atomicAdd( c.work_counter, 1u );
+            t = __shfl_sync( kFull, t, 0 );
+            if ( t >= total )
                 break;
+            const uint32_t i = deferred ? c.deferred[ t ] : c.lo + t;
             if ( mode == kCellsInitOnly )
             {
                 initial_cell( c, w, c.sites[ i ] );
@@ -1079,9 +1104,15 @@ namespace apo2
                 continue;
             if ( mode == kCellsNext && c.scheduled && !second_step_cell( c, i ) )
                 continue; // learned form: this cell was proposed within k, so it has one step only
-            const double4 si = c.sites[ i ];
+            const double4  si    = c.sites[ i ];
+            const uint32_t noted = err, counted = lane_id() < kCounters ? counts[ lane_id() ] : 0u;
             if ( mode == kCellsNext )
             {
+                if ( too_large<W>( c, i ) )
+                {
+                    defer_cell( c, i );
+                    continue;
+                }
                 load_cell( c, w, i, si, true, true );
                 if ( c.scheduled && lane_id() == 0 )
                     counts[ kCountSecondStep ]++;
@@ -1136,8 +1167,19 @@ namespace apo2
                     update_cell( c, w, i, si, j, sj, err );
                     if ( lane_id() == 0 )
                         counts[ kCountInsertions ]++;
+                    if ( outgrown<W>( err ) )
+                        break;
                 }
                 known = fmax( known, sphere_distance( si, sj ) );
+            }
+            if ( outgrown<W>( err ) )
+            {
+                err = noted;
+                __syncwarp();
+                if ( lane_id() < kCounters )
+                    counts[ lane_id() ] = counted;
+                defer_cell( c, i );
+                continue;
             }
             if ( !done )
                 done = gt_eps( known, 2.0 * cell_radius( c, w, si ) );
@@ -1170,7 +1212,8 @@ namespace apo2
     {
         extern __shared__ __align__( 16 ) unsigned char smem[];
         const uint32_t warp = threadIdx.x >> 5;
-        WarpCell<Fp32> w = carve<Fp32>( smem, warp, 0 );
+        using W = WarpCell<Fp32>;
+        W              w = carve<W>( smem, warp, 0 );
         uint32_t       err  = 0;
         while ( true )
         {
@@ -1229,7 +1272,8 @@ namespace apo2
     // -----------------------------------------------------------------------------------
     // Vertex validation (algorithm.inl:208-476)
     // -----------------------------------------------------------------------------------
-    template<bool Fp32>
+    // Over the tasks; small slots as in k_cells.
+    template<bool Fp32, bool Small>
     __global__ void __launch_bounds__( kCellBlock, 4 ) k_vertex_validation( CellContext c, const uint32_t * __restrict__ tasks,
                                                                         const uint32_t * __restrict__ task_count )
     {
@@ -1238,7 +1282,8 @@ namespace apo2
         const uint32_t gwarp = blockIdx.x * ( kCellBlock / 32 ) + warp;
         const uint32_t nwarp = gridDim.x * ( kCellBlock / 32 );
         const uint32_t lane  = lane_id();
-        WarpCell<Fp32> w = carve<Fp32>( smem, warp, 0 );
+        using W = WarpCell<Fp32, Small>;
+        W              w = carve<W>( smem, warp, 0 );
         uint32_t       err   = 0;
         const uint32_t count = *task_count;
         const uint32_t n     = c.n;
@@ -1258,7 +1303,13 @@ namespace apo2
             const uint8_t  status = c.status[ i ];
             if ( status == kFullyValidated || status == kBuried )
                 continue;
-            const double4 si = c.sites[ i ];
+            const double4  si    = c.sites[ i ];
+            const uint32_t noted = err;
+            if ( too_large<W>( c, i ) )
+            {
+                defer_cell( c, i );
+                continue;
+            }
             load_cell( c, w, i, si, true, true );
             const float known = c.known_radii[ i ];
             // the walks of the first pass start at the node around everything that the cell's spheres
@@ -1409,12 +1460,22 @@ namespace apo2
                     if ( is_known( w, tj ) )
                         continue;
                     update_cell( c, w, i, si, tj, c.sites[ tj ], err );
+                    if ( outgrown<W>( err ) )
+                        break;
                 }
+                if ( outgrown<W>( err ) )
+                    break;
                 if ( changed )
                 {
                     vs = 0;
                     restarts++;
                 }
+            }
+            if ( outgrown<W>( err ) )
+            {
+                err = noted;
+                defer_cell( c, i );
+                continue;
             }
             store_cell( c, w, i, 0, err );
             // for the edge searches
@@ -1643,7 +1704,8 @@ namespace apo2
         const uint32_t gwarp = blockIdx.x * ( kCellBlock / 32 ) + warp;
         const uint32_t nwarp = gridDim.x * ( kCellBlock / 32 );
         const uint32_t lane  = lane_id();
-        WarpCell<Fp32> w = carve<Fp32>( smem, warp, 0 );
+        using W = WarpCell<Fp32>;
+        W              w = carve<W>( smem, warp, 0 );
         uint32_t       err   = 0;
         const uint32_t count = *task_count;
         const uint32_t n     = c.n;
@@ -1999,8 +2061,9 @@ namespace apo2
         extern __shared__ __align__( 16 ) unsigned char smem[];
         const uint32_t warp  = threadIdx.x >> 5;
         const uint32_t lane  = lane_id();
-        WarpCell<Fp32> w = carve<Fp32>( smem, warp, kBisectorBytes );
-        uint32_t *     bis   = reinterpret_cast<uint32_t *>( reinterpret_cast<unsigned char *>( w.u ) + sizeof( uint32_t ) * kSiteSlots );
+        using W = WarpCell<Fp32>;
+        W              w = carve<W>( smem, warp, kBisectorBytes );
+        uint32_t *     bis   = reinterpret_cast<uint32_t *>( reinterpret_cast<unsigned char *>( w.u ) + sizeof( uint32_t ) * W::kSites );
         uint32_t       err   = 0;
         const uint32_t n     = c.n;
         const uint32_t count = tasks ? *task_count : c.hi - c.lo;
@@ -2511,18 +2574,18 @@ namespace apo2
             const auto room = []( auto * kernel, bool bisector ) {
                 cudaFuncSetAttribute( kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int( cell_smem_bytes( bisector ) ) );
             };
-            room( k_cells<false>, false );
-            room( k_cells<true>, false );
+            room( k_cells<false, false>, false );
+            room( k_cells<true, false>, false );
             room( k_cells_profile<false>, false );
             room( k_cells_profile<true>, false );
-            room( k_vertex_validation<false>, false );
-            room( k_vertex_validation<true>, false );
+            room( k_vertex_validation<false, false>, false );
+            room( k_vertex_validation<true, false>, false );
             room( k_edge_validation<false>, false );
             room( k_edge_validation<true>, false );
             room( k_bisector_validation<false>, true );
             room( k_bisector_validation<true>, true );
             int per_sm = 0;
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor( &per_sm, k_cells<false>, kCellBlock, cell_smem_bytes( false ) );
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor( &per_sm, k_cells<false, false>, kCellBlock, cell_smem_bytes( false ) );
             cell_grid_slot() = sms * std::max( 1, per_sm );
         } );
         if ( cell_grid_slot() == 0 ) // an ordinal outside the table: size it for 148 SMs x 4 blocks
@@ -2553,10 +2616,26 @@ namespace apo2
             APO2_LAUNCH( "k_knn", s, k_knn<false><<<blocks, kKnnBlock, 0, s>>>( c, step ) );
     }
 
+    // Above this many cells the cell passes run with small slots first, by what the second launch over
+    // the cells that outgrow them costs. The kNN cells rarely do: 1M protein packing 70.4 -> 67.0 ms, 1M
+    // log-normal cloud 60.2 -> 57.0, 46^3 lattice 6.03 -> 5.55. In the vertex validation a few hull
+    // cells do, and the second launch lasts as long as the longest of them, 4 to 10 ms: 1M protein
+    // packing 190.5 -> 160.1 + 5.8 ms, 1M log-normal cloud 107.2 -> 95.0 + 9.9, but 61k protein 13.0 ->
+    // 10.9 + 3.8.
+    constexpr uint32_t kSmallCellsFrom = 4096, kSmallVerticesFrom = 400000;
+
     void launch_cells( const CellContext & c, uint32_t mode, cudaStream_t s )
     {
+        const bool small = c.hi - c.lo > kSmallCellsFrom;
+        const int  grid  = cell_grid( c.n );
+        if ( small )
+        {
+            cudaMemsetAsync( c.work_counter, 0, sizeof( uint32_t ), s );
+            cudaMemsetAsync( c.deferred_count, 0, sizeof( uint32_t ), s );
+            APO2_LAUNCH( "k_cells", s, ( c.fp32 ? k_cells<true, true> : k_cells<false, true> )<<<grid, kCellBlock, small_cell_smem_bytes(), s>>>( c, mode, false ) );
+        }
         cudaMemsetAsync( c.work_counter, 0, sizeof( uint32_t ), s );
-        APO2_LAUNCH( "k_cells", s, ( c.fp32 ? k_cells<true> : k_cells<false> )<<<cell_grid( c.n ), kCellBlock, cell_smem_bytes( false ), s>>>( c, mode ) );
+        APO2_LAUNCH( "k_cells", s, ( c.fp32 ? k_cells<true, false> : k_cells<false, false> )<<<grid, kCellBlock, cell_smem_bytes( false ), s>>>( c, mode, small ) );
     }
 
     void launch_cells_profile( const CellContext & c, uint32_t step, uint32_t row, uint8_t * contributed, uint8_t * certified,
@@ -2576,8 +2655,17 @@ namespace apo2
 
     void launch_vertex_validation( const CellContext & c, const uint32_t * tasks, const uint32_t * count, cudaStream_t s )
     {
+        const int grid = cell_grid( c.n );
+        if ( c.hi - c.lo > kSmallVerticesFrom )
+        {
+            cudaMemsetAsync( c.work_counter, 0, sizeof( uint32_t ), s );
+            cudaMemsetAsync( c.deferred_count, 0, sizeof( uint32_t ), s );
+            APO2_LAUNCH( "k_vertex_validation", s, ( c.fp32 ? k_vertex_validation<true, true> : k_vertex_validation<false, true> )<<<grid, kCellBlock, small_cell_smem_bytes(), s>>>( c, tasks, count ) );
+            tasks = c.deferred;
+            count = c.deferred_count;
+        }
         cudaMemsetAsync( c.work_counter, 0, sizeof( uint32_t ), s );
-        APO2_LAUNCH( "k_vertex_validation", s, ( c.fp32 ? k_vertex_validation<true> : k_vertex_validation<false> )<<<cell_grid( c.n ), kCellBlock, cell_smem_bytes( false ), s>>>( c, tasks, count ) );
+        APO2_LAUNCH( "k_vertex_validation", s, ( c.fp32 ? k_vertex_validation<true, false> : k_vertex_validation<false, false> )<<<grid, kCellBlock, cell_smem_bytes( false ), s>>>( c, tasks, count ) );
     }
 
     void launch_edge_validation( const CellContext & c, const uint32_t * tasks, const uint32_t * count, cudaStream_t s,

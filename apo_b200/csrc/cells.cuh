@@ -13,21 +13,33 @@ namespace apo2
 
     // Shared-memory slots per warp: the reference capacities plus room for the records an
     // update appends before it compacts; writes past the slots are dropped and flagged.
-    constexpr uint32_t kVertexSlots   = 192;
-    constexpr uint32_t kEdgeSlots     = 296;
-    // Slots of the cell's neighbour list: what the 57,344 bytes a block may have at four blocks per
-    // SM leave over. A cell of simple vertices with E edges has E / 3 + 2 neighbours, so only cells
-    // above 230 edges (of 264) can outgrow it; their edges are scanned instead.
-    constexpr uint32_t kSiteSlots     = 80;
-    constexpr size_t   kWarpCellBytes = ( sizeof( double4 ) + sizeof( uint4 ) ) * kVertexSlots + sizeof( uint4 ) * kEdgeSlots
-                                      + sizeof( uint32_t ) * kSiteSlots;
+    //
+    // Sites of the neighbour list: what the 57,344 bytes a block may have at four blocks per SM leave
+    // over. A cell of simple vertices with E edges has E / 3 + 2 neighbours, so only cells above
+    // 230 edges (of 264) can outgrow it; their edges are scanned instead.
+    //
+    // Small cells, nearly all (20 to 27 vertices, 31 to 40 edges on average), take part of that, which
+    // leaves the rest of the SM's 256 KB to the L1 cache: the walks' nodes, sites and stacks hit it.
+    // A cell that outgrows the small slots is done again from its start by a second launch. (64 / 96
+    // and 128 / 208 slots: vertex validation of the 1M log-normal cloud 122 and 105.5 ms, of the 1M
+    // protein packing 168 and 172 ms, against 104.9 and 165.9 ms.)
+    template<bool Small>
+    struct CellSlots
+    {
+        static constexpr uint32_t kVertices = Small ? 96 : 192;
+        static constexpr uint32_t kEdges    = Small ? 160 : 296;
+        static constexpr uint32_t kSites    = Small ? 64 : 80;
+        static constexpr size_t   kBytes    = ( sizeof( double4 ) + sizeof( uint4 ) ) * kVertices + sizeof( uint4 ) * kEdges
+                                         + sizeof( uint32_t ) * kSites;
+        static_assert( kBytes % 32 == 0, "warp cell must keep double4 alignment" );
+    };
     constexpr size_t   kBisectorBytes = sizeof( uint32_t ) * 2 * kMaxBisectors;
-    static_assert( kWarpCellBytes % 32 == 0, "warp cell must keep double4 alignment" );
 
     inline size_t cell_smem_bytes( bool bisector )
     {
-        return ( kWarpCellBytes + ( bisector ? kBisectorBytes : 0 ) ) * ( kCellBlock / 32 );
+        return ( CellSlots<false>::kBytes + ( bisector ? kBisectorBytes : 0 ) ) * ( kCellBlock / 32 );
     }
+    inline size_t small_cell_smem_bytes() { return CellSlots<true>::kBytes * ( kCellBlock / 32 ); }
 
     struct CellContext
     {
@@ -48,6 +60,8 @@ namespace apo2
         const Scene *    scene       = nullptr; // bounds and radius range of the sites
         uint32_t *       walk_scratch = nullptr; // kWalkScratchWords per warp of the exact edge pass
         uint32_t *       work_counter = nullptr; // next cell of the dynamically scheduled passes
+        uint32_t *       deferred       = nullptr; // cells that outgrew the small slots, and their number
+        uint32_t *       deferred_count = nullptr;
         // left by the vertex validation for the edge searches of the same round: the largest vertex
         // radius of each cell, and the nodes around everything that its spheres can touch (x) and
         // around everything within the general bound of its edges (y)
