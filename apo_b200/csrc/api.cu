@@ -88,6 +88,10 @@ struct apo2_handle
     uint32_t *     tasks       = nullptr;
     uint32_t *     task_counts = nullptr; // one per validation round
     uint32_t *     error       = nullptr;
+    uint32_t *     zero        = nullptr; // cleared at the start of a build: the error word, the build
+                                          // counters, the task counts and the launches' counters
+    size_t         zero_bytes  = 0;
+    uint32_t *     zero_words  = nullptr; // of these, the launches' counters
 
     SpecBuffers   spec;
     OutputBuffers out;
@@ -220,8 +224,8 @@ namespace
         h->events_used = 0;
         h->records.clear();
         record( h, 0, s );
-        cudaMemsetAsync( h->error, 0, sizeof( uint32_t ), s );
-        cudaMemsetAsync( h->cells.counters, 0, sizeof( unsigned long long ) * kCounters, s );
+        cudaMemsetAsync( h->zero, 0, h->zero_bytes, s );
+        ZeroWords z( h->zero_words );
         launch_bounds( h->input, h->input_f64, n, h->input_d4, h->partials, h->partial_count, h->bounds_counter, h->scene,
                        h->tree.sites + n, s );
         record( h, 1, s );
@@ -235,37 +239,36 @@ namespace
             // no kNN list is ever searched; the reference leaves them all empty (0xff bytes)
             cudaMemsetAsync( h->cells.knn, 0xff, sizeof( uint32_t ) * size_t( n ) * h->cells.k, s );
             record( h, 3, s );
-            launch_cells( h->cells, kCellsInitOnly, s );
+            launch_cells( h->cells, kCellsInitOnly, z, s );
         }
         for ( uint32_t step = 0; step < steps; step++ )
         {
             launch_knn( h->cells, step, s );
             if ( step == 0 )
                 record( h, 3, s );
-            launch_cells( h->cells, step == 0 ? kCellsFirst : kCellsNext, s );
+            launch_cells( h->cells, step == 0 ? kCellsFirst : kCellsNext, z, s );
         }
         if ( h->cells.scheduled )
         {
             // learned form: a second kNN step for the uncertified cells proposed beyond k
             launch_knn( h->cells, 1, s );
-            launch_cells( h->cells, kCellsNext, s );
+            launch_cells( h->cells, kCellsNext, z, s );
         }
         record( h, 4, s );
         // stop_after (parity checks): 1 after the cells, 2 + 2r / 3 + 2r after round r's passes
         const uint32_t stop   = h->options.stop_after;
         bool           halted = stop == 1;
         const uint32_t rounds = h->options.max_iterations;
-        cudaMemsetAsync( h->task_counts, 0, sizeof( uint32_t ) * ( rounds + 1 ), s );
         for ( uint32_t r = 0; r < rounds && !halted; r++ )
         {
             launch_tasks( h->cells, h->tasks, h->task_counts + r, s );
-            launch_vertex_validation( h->cells, h->tasks, h->task_counts + r, s );
+            launch_vertex_validation( h->cells, h->tasks, h->task_counts + r, z, s );
             if ( stop == 2 + 2 * r )
                 break;
             if ( h->options.edge_search == 1 )
-                launch_edge_validation( h->cells, h->tasks, h->task_counts + r, s );
+                launch_edge_validation( h->cells, h->tasks, h->task_counts + r, z, s );
             else
-                launch_edge_validation_speculative( h->cells, h->tasks, h->task_counts + r, h->spec, s );
+                launch_edge_validation_speculative( h->cells, h->tasks, h->task_counts + r, h->spec, z, s );
             halted = stop == 3 + 2 * r;
         }
         // cells still in validation after the last round (the reference leaves them as they are)
@@ -273,9 +276,9 @@ namespace
             launch_tasks( h->cells, h->tasks, h->task_counts + rounds, s );
         record( h, 5, s );
         if ( stop == 0 && h->options.edge_search == 1 )
-            launch_bisector_validation( h->cells, nullptr, nullptr, s );
+            launch_bisector_validation( h->cells, nullptr, nullptr, z, s );
         else if ( stop == 0 )
-            launch_bisector_validation_speculative( h->cells, h->spec, s );
+            launch_bisector_validation_speculative( h->cells, h->spec, z, s );
         record( h, 6, s );
         const cudaError_t err = cudaGetLastError();
         if ( err != cudaSuccess )
@@ -385,6 +388,14 @@ namespace
         hi                   = uint32_t( uint64_t( n ) * ( opt.shard_index + 1 ) / count );
     }
 
+    // The area cleared by one memset: the error word, the build's counters, a task count per round and
+    // the launches' counters (a kNN step launches the cells once, a round at most six counting kernels).
+    size_t zero_area_bytes( const apo2_options & opt )
+    {
+        return align256( 4 ) + align256( sizeof( unsigned long long ) * kCounters ) + align256( 4 * ( kMaxRounds + 1 ) )
+               + align256( 4 * ( ZeroWords::kPerRound * ( opt.max_iterations + opt.knn_steps + 2 ) + ZeroWords::kOther ) );
+    }
+
     // Device bytes of a handle for n sites (every array of the build, carved from one block;
     // the per-cell stores only for the shard's cells).
     size_t arena_bytes( uint32_t n, const apo2_options & opt, bool f64 )
@@ -405,11 +416,11 @@ namespace
         total += align256( sortBytes );
         total += align256( size_t( n ) ) + align256( 4 * size_t( n ) * opt.k ) + align256( 4 * size_t( n ) ) * 3
                  + align256( sizeof( uint4 ) * kMaxVertices * rows ) + align256( sizeof( uint4 ) * kMaxEdges * rows );
-        total += align256( 4 * size_t( n ) ) + align256( 4 * ( kMaxRounds + 1 ) ) + align256( 4 );
+        total += align256( 4 * size_t( n ) ) + zero_area_bytes( opt );
         total += align256( 4 * size_t( n ) ) * 2 + align256( 4 * scanWords * 2 ) + align256( 16 );
         total += align256( spec_bytes( n ) );
-        total += align256( walk_scratch_bytes() ) + align256( 4 );
-        total += align256( sizeof( unsigned long long ) * kCounters ) + align256( 4 * size_t( n ) ) + align256( 8 * size_t( n ) );
+        total += align256( walk_scratch_bytes( n ) ) + align256( 4 );
+        total += align256( 4 * size_t( n ) ) + align256( 8 * size_t( n ) );
         return total;
     }
 
@@ -460,8 +471,13 @@ namespace
         c.vertices        = a.take<uint4>( rows * kMaxVertices ); // rows of cells [lo, hi)
         c.edges           = a.take<uint4>( rows * kMaxEdges );
         h->tasks          = a.take<uint32_t>( n );
-        h->task_counts    = a.take<uint32_t>( kMaxRounds + 1 );
+        const size_t zeroed = a.used;
         h->error          = a.take<uint32_t>( 1 );
+        h->zero           = h->error;
+        c.counters        = a.take<unsigned long long>( kCounters );
+        h->task_counts    = a.take<uint32_t>( kMaxRounds + 1 );
+        h->zero_words     = a.take<uint32_t>( ZeroWords::kPerRound * ( opt.max_iterations + opt.knn_steps + 2 ) + ZeroWords::kOther );
+        h->zero_bytes     = a.used - zeroed;
         c.error           = h->error;
         c.scene           = h->scene;
         h->out.vcount     = a.take<uint32_t>( n );
@@ -469,11 +485,10 @@ namespace
         h->out.tile_sums  = a.take<uint32_t>( scanWords * 2 );
         h->out.totals     = a.take<uint64_t>( 2 );
         spec_carve( h->spec, a.take<char>( spec_bytes( n ) ), n );
-        c.walk_scratch    = a.take<uint32_t>( walk_scratch_bytes() / sizeof( uint32_t ) );
+        c.walk_scratch    = a.take<uint32_t>( walk_scratch_bytes( n ) / sizeof( uint32_t ) );
         c.work_counter    = a.take<uint32_t>( 1 );
         c.deferred        = h->spec.exact_tasks; // not in use while the cell passes run
         c.deferred_count  = h->spec.exact_count;
-        c.counters        = a.take<unsigned long long>( kCounters );
         c.largest         = a.take<float>( n );
         c.around          = a.take<uint2>( n );
         c.fp32            = opt.precision == APO2_PRECISION_FP32_FILTER ? 1u : 0u;

@@ -871,7 +871,7 @@ namespace apo2
     // Propose: the learned form's first step, which also runs the k-proposal network (a separate
     // instantiation, so that the plain search keeps its small register footprint).
     template<bool Propose>
-    __global__ void __launch_bounds__( kKnnBlock ) k_knn( CellContext c, uint32_t step )
+    __global__ void __launch_bounds__( kKnnBlock ) k_knn( CellContext c, uint32_t step, uint32_t lanes )
     {
         __shared__ uint32_t    s_keys[ kMaxK * kKnnBlock ];
         __shared__ float       s_dist[ kMaxK * kKnnBlock ];
@@ -885,8 +885,8 @@ namespace apo2
                 reinterpret_cast<uint32_t *>( s_net )[ t ] = reinterpret_cast<const uint32_t *>( c.proposal )[ t ];
             __syncthreads();
         }
-        const uint32_t id = blockIdx.x * blockDim.x + threadIdx.x;
-        if ( id >= c.n )
+        const uint32_t id = ( blockIdx.x * ( kKnnBlock / 32 ) + ( threadIdx.x >> 5 ) ) * lanes + lane_id();
+        if ( lane_id() >= lanes || id >= c.n )
             return;
         // learned form's second step: only the uncertified cells proposed beyond k search again
         if ( step != 0 && c.scheduled && ( !second_step_cell( c, id ) || c.status[ id ] != kInValidation ) )
@@ -2531,10 +2531,44 @@ namespace apo2
             data[ x0 + 1 ] = ex + a;
     }
 
+    // The whole scan by one block, a tile after another: up to kScanOneBlock entries three launches
+    // take longer than the eight tiles at most (6 us for any number against 2 to 5).
+    constexpr uint32_t kScanOneBlock = 8 * kScanTile;
+
+    __global__ void __launch_bounds__( kScanBlock ) k_scan_small( uint32_t * data, uint32_t n, uint64_t * total )
+    {
+        __shared__ uint32_t tile_total;
+        uint32_t            carry = 0;
+        for ( uint32_t base = 0; base < n; base += kScanTile )
+        {
+            const uint32_t x0 = base + 2 * threadIdx.x;
+            const uint32_t a  = x0 < n ? data[ x0 ] : 0u;
+            const uint32_t b  = x0 + 1 < n ? data[ x0 + 1 ] : 0u;
+            uint32_t       t  = 0;
+            const uint32_t ex = carry + block_exclusive_scan( a + b, t );
+            if ( x0 < n )
+                data[ x0 ] = ex;
+            if ( x0 + 1 < n )
+                data[ x0 + 1 ] = ex + a;
+            if ( threadIdx.x == 0 )
+                tile_total = t;
+            __syncthreads();
+            carry += tile_total;
+            __syncthreads();
+        }
+        if ( threadIdx.x == 0 )
+            *total = carry;
+    }
+
     size_t output_scan_scratch_words( uint32_t n ) { return ( n + kScanTile - 1 ) / kScanTile + 1; }
 
     void scan_exclusive( uint32_t * data, uint32_t n, uint32_t * sums, uint64_t * total, cudaStream_t s )
     {
+        if ( n <= kScanOneBlock )
+        {
+            APO2_LAUNCH( "k_scan_small", s, k_scan_small<<<1, kScanBlock, 0, s>>>( data, n, total ) );
+            return;
+        }
         const uint32_t tiles = std::max( 1u, ( n + kScanTile - 1 ) / kScanTile );
         APO2_LAUNCH( "k_tile_sums", s, k_tile_sums<<<tiles, kScanBlock, 0, s>>>( data, n, sums ) );
         APO2_LAUNCH( "k_scan_tile_sums", s, k_scan_tile_sums<<<1, kScanBlock, 0, s>>>( sums, tiles, total ) );
@@ -2592,12 +2626,6 @@ namespace apo2
             cell_grid_slot() = 148 * 4;
     }
 
-    size_t walk_scratch_bytes()
-    {
-        configure_cell_kernels();
-        return size_t( cell_grid_slot() ) * ( kCellBlock / 32 ) * kWalkScratchWords * sizeof( uint32_t );
-    }
-
     static int cell_grid( uint32_t cells )
     {
         configure_cell_kernels();
@@ -2607,13 +2635,28 @@ namespace apo2
 
     int cell_grid_blocks( uint32_t cells ) { return cell_grid( cells ); }
 
+    size_t walk_scratch_bytes( uint32_t cells )
+    {
+        return size_t( cell_grid( cells ) ) * ( kCellBlock / 32 ) * kWalkScratchWords * sizeof( uint32_t );
+    }
+
+#ifndef APO2_KNN_WARPS
+#define APO2_KNN_WARPS ( 148u * 32u )
+#endif
     void launch_knn( const CellContext & c, uint32_t step, cudaStream_t s )
     {
-        const uint32_t blocks = ( c.n + kKnnBlock - 1 ) / kKnnBlock;
+        // A warp lasts as long as its lanes' walks together, which part at every node: few sites are
+        // spread over more warps, 32 per SM, with down to 4 lanes each (1,000 sites 220 -> 130 us, 10,000
+        // 308 -> 208 us, 61,000 429 -> 412 us).
+        uint32_t lanes = 4;
+        while ( lanes < 32 && c.n > lanes * APO2_KNN_WARPS )
+            lanes *= 2;
+        const uint32_t per_block = lanes * ( kKnnBlock / 32 );
+        const uint32_t blocks    = ( c.n + per_block - 1 ) / per_block;
         if ( c.proposal && step == 0 )
-            APO2_LAUNCH( "k_knn_propose", s, k_knn<true><<<blocks, kKnnBlock, sizeof( ProposalNet ), s>>>( c, step ) );
+            APO2_LAUNCH( "k_knn_propose", s, k_knn<true><<<blocks, kKnnBlock, sizeof( ProposalNet ), s>>>( c, step, lanes ) );
         else
-            APO2_LAUNCH( "k_knn", s, k_knn<false><<<blocks, kKnnBlock, 0, s>>>( c, step ) );
+            APO2_LAUNCH( "k_knn", s, k_knn<false><<<blocks, kKnnBlock, 0, s>>>( c, step, lanes ) );
     }
 
     // Above this many cells the cell passes run with small slots first, by what the second launch over
@@ -2624,17 +2667,23 @@ namespace apo2
     // 10.9 + 3.8.
     constexpr uint32_t kSmallCellsFrom = 4096, kSmallVerticesFrom = 400000;
 
-    void launch_cells( const CellContext & c, uint32_t mode, cudaStream_t s )
+    static CellContext with_counter( CellContext c, ZeroWords & z )
     {
-        const bool small = c.hi - c.lo > kSmallCellsFrom;
-        const int  grid  = cell_grid( c.n );
+        c.work_counter = z.take();
+        return c;
+    }
+
+    void launch_cells( const CellContext & context, uint32_t mode, ZeroWords & z, cudaStream_t s )
+    {
+        CellContext c    = with_counter( context, z );
+        const bool  small = c.hi - c.lo > kSmallCellsFrom;
+        const int   grid  = cell_grid( c.n );
+        c.deferred_count  = z.take();
         if ( small )
         {
-            cudaMemsetAsync( c.work_counter, 0, sizeof( uint32_t ), s );
-            cudaMemsetAsync( c.deferred_count, 0, sizeof( uint32_t ), s );
             APO2_LAUNCH( "k_cells", s, ( c.fp32 ? k_cells<true, true> : k_cells<false, true> )<<<grid, kCellBlock, small_cell_smem_bytes(), s>>>( c, mode, false ) );
+            c = with_counter( c, z );
         }
-        cudaMemsetAsync( c.work_counter, 0, sizeof( uint32_t ), s );
         APO2_LAUNCH( "k_cells", s, ( c.fp32 ? k_cells<true, false> : k_cells<false, false> )<<<grid, kCellBlock, cell_smem_bytes( false ), s>>>( c, mode, small ) );
     }
 
@@ -2649,35 +2698,34 @@ namespace apo2
 
     void launch_tasks( const CellContext & c, uint32_t * tasks, uint32_t * count, cudaStream_t s )
     {
-        cudaMemsetAsync( count, 0, sizeof( uint32_t ), s );
         APO2_LAUNCH( "k_tasks", s, k_tasks<<<std::max( 1u, ( c.hi - c.lo + 255 ) / 256 ), 256, 0, s>>>( c.status, c.lo, c.hi, tasks, count ) );
     }
 
-    void launch_vertex_validation( const CellContext & c, const uint32_t * tasks, const uint32_t * count, cudaStream_t s )
+    void launch_vertex_validation( const CellContext & context, const uint32_t * tasks, const uint32_t * count, ZeroWords & z, cudaStream_t s )
     {
-        const int grid = cell_grid( c.n );
+        CellContext c    = with_counter( context, z );
+        const int   grid = cell_grid( c.n );
         if ( c.hi - c.lo > kSmallVerticesFrom )
         {
-            cudaMemsetAsync( c.work_counter, 0, sizeof( uint32_t ), s );
-            cudaMemsetAsync( c.deferred_count, 0, sizeof( uint32_t ), s );
+            c.deferred_count = z.take();
             APO2_LAUNCH( "k_vertex_validation", s, ( c.fp32 ? k_vertex_validation<true, true> : k_vertex_validation<false, true> )<<<grid, kCellBlock, small_cell_smem_bytes(), s>>>( c, tasks, count ) );
             tasks = c.deferred;
             count = c.deferred_count;
+            c     = with_counter( c, z );
         }
-        cudaMemsetAsync( c.work_counter, 0, sizeof( uint32_t ), s );
         APO2_LAUNCH( "k_vertex_validation", s, ( c.fp32 ? k_vertex_validation<true, false> : k_vertex_validation<false, false> )<<<grid, kCellBlock, cell_smem_bytes( false ), s>>>( c, tasks, count ) );
     }
 
-    void launch_edge_validation( const CellContext & c, const uint32_t * tasks, const uint32_t * count, cudaStream_t s,
+    void launch_edge_validation( const CellContext & context, const uint32_t * tasks, const uint32_t * count, ZeroWords & z, cudaStream_t s,
                                  SearchProof proof )
     {
-        cudaMemsetAsync( c.work_counter, 0, sizeof( uint32_t ), s );
+        const CellContext c = with_counter( context, z );
         APO2_LAUNCH( "k_edge_validation", s, ( c.fp32 ? k_edge_validation<true> : k_edge_validation<false> )<<<cell_grid( c.n ), kCellBlock, cell_smem_bytes( false ), s>>>( c, tasks, count, proof ) );
     }
 
-    void launch_bisector_validation( const CellContext & c, const uint32_t * tasks, const uint32_t * count, cudaStream_t s )
+    void launch_bisector_validation( const CellContext & context, const uint32_t * tasks, const uint32_t * count, ZeroWords & z, cudaStream_t s )
     {
-        cudaMemsetAsync( c.work_counter, 0, sizeof( uint32_t ), s );
+        const CellContext c = with_counter( context, z );
         APO2_LAUNCH( "k_bisector_validation", s, ( c.fp32 ? k_bisector_validation<true> : k_bisector_validation<false> )<<<cell_grid( c.n ), kCellBlock, cell_smem_bytes( true ), s>>>( c, tasks, count ) );
     }
 

