@@ -18,6 +18,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import weakref
 from dataclasses import dataclass, field
 
 import numpy as np
@@ -147,6 +148,17 @@ def load_library(build_if_missing: bool = True):
 def _check(status: int) -> None:
     if status != APO2_OK:
         raise Apo2Error(status, load_library().apo2_last_error_string().decode())
+
+
+def _adopt(pointer: ctypes.c_void_p, ctype, count: int) -> np.ndarray:
+    """An array of the library's (malloc'd, released with apo2_free) as numpy, without a copy: it is
+    released when the last array over it goes."""
+    if not count:
+        load_library().apo2_free(pointer)
+        return np.zeros(0, np.dtype(ctype))
+    memory = (ctype * count).from_address(pointer.value)
+    weakref.finalize(memory, load_library().apo2_free, ctypes.c_void_p(pointer.value))
+    return np.frombuffer(memory, dtype=np.dtype(ctype))
 
 
 def _as_sites(sites) -> tuple[np.ndarray, int]:
@@ -431,12 +443,7 @@ class Batch:
         out = None
         if vertices:
             total = int(voff[-1])
-            try:
-                P = np.ctypeslib.as_array(ctypes.cast(pos, ctypes.POINTER(ctypes.c_double)), shape=(max(total, 1) * 4,))[:total * 4].copy()
-                I = np.ctypeslib.as_array(ctypes.cast(ids, ctypes.POINTER(ctypes.c_uint32)), shape=(max(total, 1) * 4,))[:total * 4].copy()
-            finally:
-                self._lib.apo2_free(pos)
-                self._lib.apo2_free(ids)
+            P, I = _adopt(pos, ctypes.c_double, 4 * total), _adopt(ids, ctypes.c_uint32, 4 * total)
             out = [VertexDiagram(vertices=P[4 * int(voff[d]):4 * int(voff[d + 1])], verticesId=I[4 * int(voff[d]):4 * int(voff[d + 1])])
                    for d in range(len(arrays))]
         return out, counts, ms
@@ -456,14 +463,8 @@ def computeApolloniusDiagram(sites) -> VertexDiagram:
     a, dtype = _as_sites(sites)
     pos, ids, count = ctypes.c_void_p(), ctypes.c_void_p(), ctypes.c_uint64()
     _check(lib.apo2_compute_diagram(a.ctypes.data, a.shape[0], dtype, ctypes.byref(pos), ctypes.byref(ids), ctypes.byref(count)))
-    try:
-        n = count.value
-        p = np.ctypeslib.as_array(ctypes.cast(pos, ctypes.POINTER(ctypes.c_double)), shape=(4 * n,)).copy() if n else np.zeros(0)
-        i = np.ctypeslib.as_array(ctypes.cast(ids, ctypes.POINTER(ctypes.c_uint32)), shape=(4 * n,)).copy() if n else np.zeros(0, np.uint32)
-    finally:
-        lib.apo2_free(pos)
-        lib.apo2_free(ids)
-    return VertexDiagram(vertices=p, verticesId=i)
+    return VertexDiagram(vertices=_adopt(pos, ctypes.c_double, 4 * count.value),
+                         verticesId=_adopt(ids, ctypes.c_uint32, 4 * count.value))
 
 
 def fma_peak() -> tuple[float, float]:

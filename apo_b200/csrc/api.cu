@@ -1640,9 +1640,32 @@ namespace
         delete b;
     }
 
+    // One diagram's vertices on the host, not written before the copy from the device.
+    struct HostVertices
+    {
+        double4 * pos = nullptr;
+        uint4 *   ids = nullptr;
+        HostVertices() = default;
+        HostVertices( const HostVertices & ) = delete;
+        HostVertices & operator=( const HostVertices & ) = delete;
+        ~HostVertices() { release(); }
+        bool allocate( uint64_t count )
+        {
+            pos = static_cast<double4 *>( std::malloc( sizeof( double4 ) * count ) );
+            ids = static_cast<uint4 *>( std::malloc( sizeof( uint4 ) * count ) );
+            return pos && ids;
+        }
+        void release()
+        {
+            std::free( pos );
+            std::free( ids );
+            pos = nullptr;
+            ids = nullptr;
+        }
+    };
+
     // One diagram on one worker: upload, build, extract, counts (and the vertices when asked).
-    apo2_status batch_one( apo2_batch::Worker & w, const float * sites, uint32_t n, bool want_vertices,
-                           std::vector<double4> & pos, std::vector<uint4> & ids, uint64_t & count, float & ms )
+    apo2_status batch_one( apo2_batch::Worker & w, const float * sites, uint32_t n, HostVertices * out, uint64_t & count, float & ms )
     {
         apo2_handle * h = w.h;
         if ( !carve( h, n ) )
@@ -1667,12 +1690,12 @@ namespace
         count = w.words[ 0 ];
         if ( count > h->out.vcap )
             return fail( APO2_ERR_CAPACITY, "batch output capacity" );
-        if ( want_vertices && count )
+        if ( out && count )
         {
-            pos.resize( count );
-            ids.resize( count );
-            APO2_CUDA( cudaMemcpyAsync( pos.data(), h->out.vpos, sizeof( double4 ) * count, cudaMemcpyDeviceToHost, w.s ), "batch output" );
-            APO2_CUDA( cudaMemcpyAsync( ids.data(), h->out.vids, sizeof( uint4 ) * count, cudaMemcpyDeviceToHost, w.s ), "batch output" );
+            if ( !out->allocate( count ) )
+                return fail( APO2_ERR_OUT_OF_MEMORY, "batch output (host)" );
+            APO2_CUDA( cudaMemcpyAsync( out->pos, h->out.vpos, sizeof( double4 ) * count, cudaMemcpyDeviceToHost, w.s ), "batch output" );
+            APO2_CUDA( cudaMemcpyAsync( out->ids, h->out.vids, sizeof( uint4 ) * count, cudaMemcpyDeviceToHost, w.s ), "batch output" );
             APO2_CUDA( cudaStreamSynchronize( w.s ), "batch output" );
         }
         APO2_CUDA( cudaEventElapsedTime( &ms, w.e0, w.e1 ), "batch timing" );
@@ -1765,8 +1788,7 @@ apo2_status apo2_batch_build( apo2_batch * b, const float * sites_xyzr, const ui
     std::stable_sort( order.begin(), order.end(), [ & ]( uint32_t x, uint32_t y ) {
         return site_offsets[ x + 1 ] - site_offsets[ x ] > site_offsets[ y + 1 ] - site_offsets[ y ];
     } );
-    std::vector<std::vector<double4>> pos( want ? count : 0 );
-    std::vector<std::vector<uint4>>   idv( want ? count : 0 );
+    std::vector<HostVertices>         vertices( want ? count : 0 );
     std::vector<uint64_t>             counts( count, 0 );
     std::vector<float>                times( count, 0.f );
     std::atomic<uint32_t>             next { 0 };
@@ -1774,8 +1796,6 @@ apo2_status apo2_batch_build( apo2_batch * b, const float * sites_xyzr, const ui
     std::mutex                        error_mutex;
     apo2_status                       first_status = APO2_OK;
     std::string                       first_error;
-    std::vector<double4>              no_pos;
-    std::vector<uint4>                no_ids;
 
     auto run = [ & ]( apo2_batch::Worker & w ) {
         cudaSetDevice( b->device );
@@ -1786,9 +1806,7 @@ apo2_status apo2_batch_build( apo2_batch * b, const float * sites_xyzr, const ui
                 break;
             const uint32_t d  = order[ k ];
             const uint32_t n  = uint32_t( site_offsets[ d + 1 ] - site_offsets[ d ] );
-            std::vector<double4> & p = want ? pos[ d ] : no_pos;
-            std::vector<uint4> &   q = want ? idv[ d ] : no_ids;
-            const apo2_status st = batch_one( w, sites_xyzr + 4 * site_offsets[ d ], n, want, p, q, counts[ d ], times[ d ] );
+            const apo2_status st = batch_one( w, sites_xyzr + 4 * site_offsets[ d ], n, want ? &vertices[ d ] : nullptr, counts[ d ], times[ d ] );
             if ( st != APO2_OK )
             {
                 std::lock_guard<std::mutex> lock( error_mutex );
@@ -1826,13 +1844,30 @@ apo2_status apo2_batch_build( apo2_batch * b, const float * sites_xyzr, const ui
             std::free( I );
             return fail( APO2_ERR_OUT_OF_MEMORY, "batch output (host)" );
         }
-        for ( uint32_t d = 0; d < count; d++ )
+        // gathered by as many threads as built them: most of it is the first touch of the pages
+        std::atomic<uint32_t> gathered { 0 };
+        auto                  gather = [ & ] {
+            for ( uint32_t d = gathered.fetch_add( 1 ); d < count; d = gathered.fetch_add( 1 ) )
+                if ( counts[ d ] )
+                {
+                    std::memcpy( P + 4 * vertex_offsets[ d ], vertices[ d ].pos, sizeof( double4 ) * counts[ d ] );
+                    std::memcpy( I + 4 * vertex_offsets[ d ], vertices[ d ].ids, sizeof( uint4 ) * counts[ d ] );
+                    vertices[ d ].release();
+                }
+        };
+        threads.clear();
+        try
         {
-            if ( !counts[ d ] )
-                continue;
-            std::memcpy( P + 4 * vertex_offsets[ d ], pos[ d ].data(), sizeof( double4 ) * counts[ d ] );
-            std::memcpy( I + 4 * vertex_offsets[ d ], idv[ d ].data(), sizeof( uint4 ) * counts[ d ] );
+            for ( size_t t = 1; t < b->workers.size(); t++ )
+                threads.emplace_back( gather );
         }
+        catch ( const std::exception & )
+        {
+            // fewer threads gather
+        }
+        gather();
+        for ( auto & t : threads )
+            t.join();
         *positions = P;
         *ids       = I;
     }
