@@ -152,12 +152,12 @@ def _check(status: int) -> None:
 
 def _adopt(pointer: ctypes.c_void_p, ctype, count: int) -> np.ndarray:
     """An array of the library's (malloc'd, released with apo2_free) as numpy, without a copy: it is
-    released when the last array over it goes."""
+    released when the last array over it goes (at exit with the process: arrays may outlive exit handlers)."""
     if not count:
         load_library().apo2_free(pointer)
         return np.zeros(0, np.dtype(ctype))
     memory = (ctype * count).from_address(pointer.value)
-    weakref.finalize(memory, load_library().apo2_free, ctypes.c_void_p(pointer.value))
+    weakref.finalize(memory, load_library().apo2_free, ctypes.c_void_p(pointer.value)).atexit = False
     return np.frombuffer(memory, dtype=np.dtype(ctype))
 
 
