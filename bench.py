@@ -51,15 +51,13 @@ PEAKS_FALLBACK = {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0}
 C_QUAD = 216
 C_TEST = 11
 
-# DRAM bytes (read + write) per site of one launch, by kernel, from one-kernel ncu captures (--set
-# full, the kernel's first launch), scaled by the sites processed: the log-normal cloud of 1M sites
-# at the evaluation density for the edge-search kernels, the protein-like packing of 100,000 sites
-# for the others.
-TRAFFIC_BYTES_PER_SITE = {"k_edge_heavy_sub": (22334.4, "1M log-normal capture"),
-                          "k_edge_speculate": (1418.2, "1M log-normal capture"),
-                          "k_vertex_validation": (1839.3, "100k protein-like capture"),
-                          "k_cells": (316.6, "100k protein-like capture"),
-                          "k_bisector_validation": (1054.6, "100k protein-like capture")}
+# DRAM bytes (read + write) per site of one launch, by kernel, from ncu captures of the kernel's first
+# launch on the log-normal cloud of 300,000 sites at the evaluation density, scaled by the sites
+# processed. The other kernels have no capture.
+TRAFFIC_BYTES_PER_SITE = {"k_vertex_validation": (1643.8, "300k log-normal capture"),
+                          "k_edge_cells": (1430.7, "300k log-normal capture"),
+                          "k_cells": (528.8, "300k log-normal capture"),
+                          "k_edge_speculate": (134.4, "300k log-normal capture")}
 
 
 def measure_fp64_peak(device) -> float:
