@@ -160,6 +160,13 @@ namespace apo2
 #define APO2_EXACT_LANE_WALK 256
 #endif
     constexpr uint32_t kLaneWalk         = APO2_EXACT_LANE_WALK;
+    // After the edge-parallel search a cell has few edges left to search, and a warp whose few walking
+    // lanes go one node per step, each candidate stopping them all, takes longer than the same searches
+    // one after another by the whole warp: they go there after 4 steps (longest launches of the pass
+    // summed over the rounds, 256 -> 32 -> 4 steps: 100,000 uniform sites 5.4 -> 2.6 -> 1.8 ms, 10,000 0.42 ->
+    // 0.29 -> 0.26, 300,000 log-normal 3.9 -> 3.7 -> 3.6, 800,000 8.2 -> 8.6 -> 8.2, 1M protein-like 1.1 ->
+    // 0.6 -> 0.6). Without that search every edge walks, 32 at a time, and lanes keep kLaneWalk.
+    constexpr uint32_t kLaneWalkLeft     = 4;
 #ifndef APO2_COOP_WIDTH
 #define APO2_COOP_WIDTH 4
 #endif
