@@ -199,14 +199,13 @@ namespace apo2
         bool     covered; // the reach lies in what the cell's vertex spheres can touch
     };
 
-    // Bounding volume of edge (k, l) of cell i and the security-radius test
-    // (algorithm.inl:555-614). Returns false when the edge needs no search.
-    __device__ __forceinline__ bool setup_edge( const CellContext & c, EdgeSearch & s, float known )
+    // Bounding volume of edge (k, l) of cell i (algorithm.inl:555-600); the trisector's roots are
+    // left in ev0 and ev1. Returns whether it is an ellipse.
+    __device__ __forceinline__ bool bound_edge( EdgeSearch & s, double4 & ev0, double4 & ev1 )
     {
-        uint32_t type = 0;
-        double4  ev0 = make_double4( 0, 0, 0, 0 ), ev1 = make_double4( 0, 0, 0, 0 );
-        type          = trisector( s.si, s.sk, s.sl, ev0, ev1 );
-        s.hyperbola   = type == 1;
+        ev0 = ev1 = make_double4( 0, 0, 0, 0 );
+        const uint32_t type = trisector( s.si, s.sk, s.sl, ev0, ev1 );
+        s.hyperbola         = type == 1;
         const bool   ellipse = type == 2;
         const float4 v1 = to_float( ev0 ), v2 = to_float( ev1 );
         s.planes.n1 = s.planes.n2 = s.planes.p1 = s.planes.p2 = make_float3( 0, 0, 0 );
@@ -231,12 +230,19 @@ namespace apo2
             s.planes.p1      = to_float( p1 );
             s.planes.p2      = to_float( p4 );
         }
-        const float4 fsi    = to_float( s.si );
-        const bool   inside = lt_eps( flength( f3( fsi ) - f3( s.bsph ) ), known - s.bsph.w );
-        if ( inside )
-            return false;
+        return ellipse;
+    }
 
-        // reach of the search: the arc's ends and its largest radius
+    // Does the security radius cover the edge (algorithm.inl:601-614)? Then it needs no search.
+    __device__ __forceinline__ bool covers_edge( const EdgeSearch & s, float known )
+    {
+        return lt_eps( flength( f3( to_float( s.si ) ) - f3( s.bsph ) ), known - s.bsph.w );
+    }
+
+    // Reach of the search of a bounded edge: the arc's ends and its largest radius.
+    __device__ __forceinline__ void reach_edge( const CellContext & c, EdgeSearch & s, bool ellipse, double4 ev0, double4 ev1 )
+    {
+        const float4 fsi = to_float( s.si );
         ArcEnds ends;
         double  wmax = stored_ends( c, s.i, s.si, s.k, s.l, ends, s.hint );
         if ( ellipse || s.closed )
@@ -282,7 +288,6 @@ namespace apo2
         for ( uint32_t h = 0; h < 2; h++ )
             if ( s.hint[ h ] != kNone && !in_sorted( s.nbr, s.nbr_count, s.hint[ h ] ) )
                 s.hint[ h ] = kNone;
-        return true;
     }
 
     // The walk is bound by the node steps (two boxes against three balls and two planes, 50 to 90
@@ -385,7 +390,12 @@ namespace apo2
             return false;
         s.sk = c.sites[ s.k ];
         s.sl = c.sites[ s.l ];
-        return setup_edge( c, s, c.known_radii[ s.i ] );
+        double4    ev0, ev1;
+        const bool ellipse = bound_edge( s, ev0, ev1 );
+        if ( covers_edge( s, c.known_radii[ s.i ] ) )
+            return false;
+        reach_edge( c, s, ellipse, ev0, ev1 );
+        return true;
     }
 
     // Edges of cells with few surroundings, nearly all: a warp per cell collects the sites, other than
@@ -665,6 +675,9 @@ namespace apo2
         return kWalkDone;
     }
 
+    // The search of a listed edge. Whether the security radius covers it was decided where it was
+    // listed and is not asked again: that compares floats near a threshold, and another copy of the
+    // code may round them the other way.
     __device__ __forceinline__ void search_of_heavy( const CellContext & c, const uint32_t * tasks, const SpecBuffers & b,
                                                      uint2 h, EdgeSearch & s )
     {
@@ -680,7 +693,9 @@ namespace apo2
         s.sl          = c.sites[ s.l ];
         s.nbr         = b.nbr + size_t( s.t ) * kNbrCap;
         s.nbr_count   = b.nbr_count[ s.t ];
-        setup_edge( c, s, c.known_radii[ s.i ] ); // the lane path already found it needs a search
+        double4    ev0, ev1;
+        const bool ellipse = bound_edge( s, ev0, ev1 );
+        reach_edge( c, s, ellipse, ev0, ev1 );
     }
 
     __global__ void __launch_bounds__( kHeavyBlock, 4 ) k_edge_heavy( CellContext c, const uint32_t * __restrict__ tasks,
