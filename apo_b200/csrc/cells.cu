@@ -75,18 +75,6 @@ namespace apo2
     __device__ __forceinline__ uint32_t estatus( uint4 r ) { return r.w & 0xffu; }
 
 
-    // The sites the emptiness and known-neighbour tests range over, those of the cell's edges, as a
-    // sequence. The neighbour list holds each once (an edge list names every neighbour about six
-    // times); a cell with more neighbours than slots goes by its edges.
-    struct SiteSequence
-    {
-        const uint32_t * words;
-        uint32_t         count, shift; // shift 0: a list of ids; 1: two ids at the front of 16-byte records
-        __device__ __forceinline__ uint32_t operator[]( uint32_t q ) const
-        {
-            return words[ ( ( q >> shift ) << ( 2 * shift ) ) + ( q & shift ) ];
-        }
-    };
     template<class W>
     __device__ __forceinline__ SiteSequence sites_of( const W & w )
     {
@@ -1515,16 +1503,6 @@ namespace apo2
         double4  sk, sl;
     };
 
-    __device__ __forceinline__ float3 shfl3( float3 v, uint32_t src )
-    {
-        return make_float3( __shfl_sync( kFull, v.x, src ), __shfl_sync( kFull, v.y, src ), __shfl_sync( kFull, v.z, src ) );
-    }
-    __device__ __forceinline__ float4 shfl4f( float4 v, uint32_t src )
-    {
-        return make_float4( __shfl_sync( kFull, v.x, src ), __shfl_sync( kFull, v.y, src ), __shfl_sync( kFull, v.z, src ),
-                            __shfl_sync( kFull, v.w, src ) );
-    }
-
     // The rest of a long edge search, walked by the whole warp in the lane walk's order.
     // The walk has no running bound: which children of a node are entered, and in which order
     // (closer first), depends on the node alone, so its leaves come in one fixed order and the
@@ -1831,7 +1809,11 @@ namespace apo2
                                 wmax = fmax( wmax, apex[ a ].w );
                         }
                     }
-                    reach = edge_reach( c, si, sk, sl, hyperbola, ends, wmax, bsph );
+                    const bool bounded = ends.count == 2 && known_by_lane( w, ends.m[ 0 ] ) && known_by_lane( w, ends.m[ 1 ] );
+                    OpenEnds   open;
+                    reach = edge_reach( c, si, sk, sl, hyperbola, ends, bounded, wmax, bsph, open );
+                    close_ends( c, si, k, l, ends, sites_of( w ), open, reach );
+                    settle( reach, open );
                 }
 
                 // proven free of contributors on this very cell state

@@ -195,6 +195,18 @@ namespace apo2
         return ( r.w & 0xffu ) ? x[ 1 ] : x[ 0 ];
     }
 
+    // The sites the emptiness and known-neighbour tests range over, those of the cell's edges, as a
+    // sequence. The neighbour list holds each once (an edge list names every neighbour about six
+    // times); a cell with more neighbours than slots goes by its edges.
+    struct SiteSequence
+    {
+        const uint32_t * words;
+        uint32_t         count, shift; // shift 0: a list of ids; 1: two ids at the front of 16-byte records
+        __device__ __forceinline__ uint32_t operator[]( uint32_t q ) const
+        {
+            return words[ ( ( q >> shift ) << ( 2 * shift ) ) + ( q & shift ) ];
+        }
+    };
     // ---------------------------------------------------------------------------------
     // Reach of an edge search. A site j contributes to edge (k, l) of cell i only through a
     // root x that passes the emptiness test against the cell's neighbours, i.e. a point of
@@ -208,27 +220,35 @@ namespace apo2
     //
     // That bound is kReachBall: one ball around c_i, |c_j - c_i| <= 2 w + r_i + r_max, or the
     // reference's own bounding sphere where that is smaller. Between two vertices the spheres along
-    // the arc lie in three far smaller balls (arc_reach).
+    // the arc lie in three far smaller balls, and arc_reach shows for each edge that the rest of the
+    // trisector is closed by neighbours of the cell, whichever vertices the cell has or lacks: with
+    // duplicate sites, and where roots went lost to rounding, a cell lacks some, and an arc between two
+    // of the others is not all that is open.
     //
-    // One kind of contributor lies outside them: a root so far away that the single-precision
-    // lengths of the emptiness test cannot tell the neighbours apart (its radius is 7e7 and more
-    // where it happened, once in some ten builds, on edges of hull cells). The reference
-    // takes such a root, so it has to be found. It belongs to a site that touches a plane tangent to
-    // the edge's three sites, so on a hyperbolic trisector the boxes that reach one of the two planes
-    // within the general bound are entered too (kReachArcPlanes); an elliptic one has no
-    // point further than its apex. Most planes are out, though (far_roots_blocked).
+    // One kind of contributor lies outside the balls all the same.
+    //
+    // A root so far away that the single-precision lengths of the emptiness test cannot tell the
+    // neighbours apart (its radius was 7e7 and more where it happened, once in some ten builds, on edges
+    // of hull cells). The reference takes such a root, so it has to be found. A neighbour that stands out by h
+    // beyond the tangent plane conflicts by about as much with every root there, which rounding hides
+    // from a radius of h / 4e-7 on: `far`, at most kFarRoot. From there on a site of such a root touches the
+    // plane, so on a hyperbolic trisector the boxes that reach one of the two planes within the general
+    // bound are entered too (kReachArcPlanes); an elliptic one has no point further than its apex. Most
+    // planes are out, though (far_roots_blocked).
     // ---------------------------------------------------------------------------------
     constexpr uint32_t kReachBall = 0, kReachArc = 1, kReachArcPlanes = 2;
     constexpr double   kFarRoot   = 2.5e5; // radius from which a root counts as far: single precision is off by 0.1 there
+    constexpr float    kFarOut    = 2.5e6f; // ... by 4e-7 of the radius: least radius, by the depth of the conflict
 
     struct EdgeReach
     {
         float4   ball[ 3 ]; // kReachBall: the same one three times
-        float4   limit;     // kReachArcPlanes: ball holding every site that the planes let in
-        float    slab[ 2 ]; // and how near to each plane it has to come
+        float4   limit;     // ball holding every site that the planes let in
+        float    slab[ 2 ]; // kReachArcPlanes: how near to each tangent plane it has to come
         // hyperbolic trisectors: a contributor lies wholly below both planes (algorithm.inl:695-700), so
         // a box has to go below them by a smallest sphere's diameter; less this rounding margin
         float    diameter, margin;
+        float    far; // kReachArcPlanes: least radius of a far root
         bool     below;
         uint32_t kind;
     };
@@ -271,18 +291,23 @@ namespace apo2
     }
     // May box or site `x` be, or hold, a contributor? The balls are tested without branches: a walk's
     // lanes would take them all the same.
-    template<class X>
+    template<bool Limited = true, class X>
     __device__ __forceinline__ bool within( const EdgeReach & a, const TangentPlanes & t, const X & x )
     {
-        bool in = meets( a.ball[ 0 ], x ) | meets( a.ball[ 1 ], x ) | meets( a.ball[ 2 ], x );
+        bool in   = meets( a.ball[ 0 ], x ) | meets( a.ball[ 1 ], x ) | meets( a.ball[ 2 ], x );
+        bool more = false;
         if ( a.below )
         {
             const float2 h1 = heights( t.n1, t.p1, a.diameter, x ), h2 = heights( t.n2, t.p2, a.diameter, x );
             if ( a.kind == kReachArcPlanes )
-                in = in | ( ( ( h1.y >= -a.slab[ 0 ] ) | ( h2.y >= -a.slab[ 1 ] ) ) & meets( a.limit, x ) );
-            in = in & ( h1.x < a.margin ) & ( h2.x < a.margin );
+                more = more | ( h1.y >= -a.slab[ 0 ] ) | ( h2.y >= -a.slab[ 1 ] );
+            if ( Limited )
+                more = more & meets( a.limit, x );
+            return ( in | more ) & ( h1.x < a.margin ) & ( h2.x < a.margin );
         }
-        return in;
+        if ( Limited )
+            more = more & meets( a.limit, x );
+        return in | more;
     }
 
     // Does neighbour m conflict with every far root beyond the plane of outward normal n? Its
@@ -290,11 +315,11 @@ namespace apo2
     // precision alike: where m is the nearer one it does not come out farther, and the test of m
     // against the root's radius, re-measured from c_i, is decided by the larger radius of m. (The
     // approximate root falls between neighbouring floats at 508 of the 2^31 positive ones.)
-    __device__ __forceinline__ bool far_roots_blocked( float3 n, float4 fi, float4 m )
+    __device__ __forceinline__ bool far_roots_blocked( float3 n, float4 fi, float4 m, float far )
     {
         const float3 e  = f3( m ) - f3( fi );
         const float  ee = fdot( e, e );
-        return m.w >= fi.w + 1e-3f && fdot( n, e ) >= 5e-3f * sqrtf( ee ) + float( 1.0 / kFarRoot ) * ee;
+        return m.w >= fi.w + 1e-3f && fdot( n, e ) >= 5e-3f * sqrtf( ee ) + ee / far;
     }
 
     // The ball with its margins: 1 % and 1e-3 as the reach always had, and the rounding of a far
@@ -361,30 +386,45 @@ namespace apo2
                 count++;
             }
         }
-        double wmax = 0.0;
+        double   wmax = 0.0;
+        uint32_t v    = at[ 0 ];
 #pragma unroll 1
-        for ( uint32_t q = 0; q < 2; q++ )
+        while ( v < vn ) // hardly ever more than two
         {
-            const uint32_t v = q ? at[ 1 ] : at[ 0 ];
-            if ( v < vn )
+            const uint4   r = store[ v ];
+            const double4 x = solve_vertex( c, si, r );
+            wmax            = fmax( wmax, x.w );
+            ends.add( x, third_site( r, k, l ) );
+            if ( v == at[ 0 ] )
+                v = at[ 1 ];
+            else
             {
-                const uint4   r = store[ v ];
-                const double4 x = solve_vertex( c, si, r );
-                wmax            = fmax( wmax, x.w );
-                ends.add( x, third_site( r, k, l ) );
-            }
-        }
-        for ( uint32_t v = more; v < vn; v++ ) // more than two: rare
-        {
-            const uint4 r = store[ v ];
-            if ( vertex_on_edge( r, k, l ) )
-            {
-                wmax = fmax( wmax, solve_vertex( c, si, r ).w );
-                ends.count++;
+                v = v == at[ 1 ] ? more : v + 1;
+                while ( v < vn && !vertex_on_edge( store[ v ], k, l ) )
+                    v++;
             }
         }
         return wmax;
     }
+
+    __device__ __forceinline__ float4 neighbour( const CellContext & c, uint32_t u ) { return u < c.n ? c.sites_f[ u ] : to_float( c.sites[ u ] ); }
+
+    // Where the conflict of an end's third site ends again, further out: the point and its radius, what the
+    // curve goes on to (a hyperbola to infinity, in a direction; an ellipse to a point half-way round to
+    // the other end, with its radius), and the least radius on the way.
+    struct OpenEnds
+    {
+        float4   at[ 2 ], away[ 2 ];
+        float    low[ 2 ];
+        uint32_t mask = 0;
+        __device__ __forceinline__ void add( int a, float3 x, float w, float3 on, float on_w, float least )
+        {
+            ( a ? at[ 1 ] : at[ 0 ] )     = make_float4( x.x, x.y, x.z, w );
+            ( a ? away[ 1 ] : away[ 0 ] ) = make_float4( on.x, on.y, on.z, on_w );
+            ( a ? low[ 1 ] : low[ 0 ] )   = least;
+            mask |= 1u << a;
+        }
+    };
 
     // The balls of the arc of trisector (i, k, l) between its two vertices. With c_i as the origin,
     // e_k = c_k - c_i, d_k = r_k - r_i and rho = w + r_i = |x|, the trisector's points are
@@ -399,10 +439,12 @@ namespace apo2
     // the sphere (or of a box around it) from x: a ball of radius sqrt(w^2 + D). (With equal radii
     // it passes through the three centres, in the union of the other two: only unequal radii
     // leave anything to find.) On a hyperbola (of which the points with rho > 0 are one branch) the
-    // arc is the one between the ends; on an ellipse it is the smaller one if on both ends the
-    // third site's conflict fades that way. False where the points do not determine this safely.
-    __device__ __forceinline__ bool arc_reach( const CellContext & c, double4 si, double4 sk, double4 sl, const ArcEnds & ends,
-                                               EdgeReach & reach )
+    // arc is the piece between the ends, on an ellipse the smaller one, if at both ends the third
+    // site's conflict fades that way. (It does not in a cell that has one of two equal sites twice:
+    // both its vertices on an edge may be the same point, and the rest of the arc is open.) False
+    // where the points do not determine this safely.
+    __device__ __forceinline__ bool arc_reach( const CellContext & c, double4 si, double4 sk, double4 sl,
+                                               const ArcEnds & ends, OpenEnds & open, EdgeReach & reach )
     {
         const double3 o   = d3( si );
         const double3 ek  = d3( sk ) - o, el = d3( sl ) - o;
@@ -425,64 +467,248 @@ namespace apo2
         if ( !( ddot( off0, off0 ) <= 1e-8 * ( 1.0 + rho0 ) * ( 1.0 + rho0 )
                 && ddot( off1, off1 ) <= 1e-8 * ( 1.0 + rho1 ) * ( 1.0 + rho1 ) && fmax( rho0, rho1 ) < 1e9 ) )
             return false;
-        const double slack = 1e-3 * ( 1.0 + fabs( s0 ) + fabs( s1 ) );
-        double       sT = s0, rhoT = rho0;
+        // the curve at the ends, in one direction along it, and how far the second end lies ahead of the first
+        double2 along0, along1;
+        double  ahead, near; // ends less than `near` apart coincide
+        double  sT = s0, rhoT = rho0;
+        double  rc = 0.0, ar = 0.0, as = 0.0; // ellipse: centre and axes, and the ends on its unit circle
+        double2 c0 = make_double2( 0, 0 ), c1 = make_double2( 0, 0 );
         if ( alpha > 1e-6 )
         {
             // s_a s + (beta - alpha rho_a) rho = -(beta rho_a + gamma) is the tangent at end a
             const double m0 = beta - alpha * rho0, m1 = beta - alpha * rho1;
             const double h0 = -( beta * rho0 + gamma ), h1 = -( beta * rho1 + gamma );
-            const double meet = s0 * m1 - s1 * m0;
-            if ( fabs( s0 - s1 ) >= 1e-3 * slack ) // else the ends coincide
+            const double meet  = s0 * m1 - s1 * m0;
+            const double slack = 1e-3 * ( 1.0 + fabs( s0 ) + fabs( s1 ) );
+            near               = 1e-3 * slack;
+            if ( fabs( s0 - s1 ) >= near )
             {
                 sT   = ( h0 * m1 - h1 * m0 ) / meet;
                 rhoT = ( s0 * h1 - s1 * h0 ) / meet;
             }
-            if ( !( sT >= fmin( s0, s1 ) - slack && sT <= fmax( s0, s1 ) + slack && rhoT >= -1e-3
+            if ( !( m0 < 0.0 && m1 < 0.0 && sT >= fmin( s0, s1 ) - slack && sT <= fmax( s0, s1 ) + slack && rhoT >= -1e-3
                     && rhoT <= 1.001 * fmax( rho0, rho1 ) + 1e-3 ) )
                 return false;
+            along0     = make_double2( s0, -m0 );
+            along1     = make_double2( s1, -m1 );
+            ahead      = s1 - s0;
             reach.kind = kReachArcPlanes;
         }
         else if ( alpha < -1e-6 && beta * beta + alpha * gamma > 0.0 )
         {
-            // (rho, s) = centre + (ar cos, as sin); c0 and c1 the unit vectors of the ends
-            const double disc = beta * beta + alpha * gamma, rc = beta / alpha;
-            const double ar = sqrt( disc ) / -alpha, as = sqrt( disc / -alpha );
+            // (rho, s) = (rc + ar cos, as sin)
+            const double disc = beta * beta + alpha * gamma;
+            rc                = beta / alpha;
+            ar                = sqrt( disc ) / -alpha;
+            as                = sqrt( disc / -alpha );
             if ( !( rc + ar < kFarRoot ) )
                 return false;
-            const double2 c0 = make_double2( ( rho0 - rc ) / ar, s0 / as ), c1 = make_double2( ( rho1 - rc ) / ar, s1 / as );
+            c0                  = make_double2( ( rho0 - rc ) / ar, s0 / as );
+            c1                  = make_double2( ( rho1 - rc ) / ar, s1 / as );
             const double  cosine = ddot( c0, c1 );
             if ( !( cosine > -.5 && fabs( ddot( c0, c0 ) - 1.0 ) < 1e-3 && fabs( ddot( c1, c1 ) - 1.0 ) < 1e-3 ) )
                 return false; // more than a third of the ellipse apart
-            for ( int a = 0; a < 2; a++ )
-            {
-                // the linear form of the third site grows from this end towards the other
-                const double4 sm = c.sites[ a ? ends.m[ 1 ] : ends.m[ 0 ] ];
-                const double3 em = d3( sm ) - o;
-                const double2 from = a ? c1 : c0, to = a ? c0 : c1;
-                const double  dr = ar * ( to.x - cosine * from.x ), ds = as * ( to.y - cosine * from.y );
-                const double  fr = ddot( em, B ) + ( sm.w - si.w ), fs = ddot( em, n );
-                if ( !( -( fr * dr + fs * ds ) > 1e-3 * ( fabs( fr * dr ) + fabs( fs * ds ) ) ) )
-                    return false;
-            }
+            along0     = make_double2( -ar * c0.y, as * c0.x );
+            along1     = make_double2( -ar * c1.y, as * c1.x );
+            ahead      = c0.x * c1.y - c0.y * c1.x;
+            near       = 1e-6;
             rhoT       = rc + ar * ( c0.x + c1.x ) / ( 1.0 + cosine );
             sT         = as * ( c0.y + c1.y ) / ( 1.0 + cosine );
             reach.kind = kReachArc;
         }
         else
             return false;
+        // Is every root of the cell in the piece between the ends? Each end's third site, a neighbour, has to
+        // conflict from its end on outward, and the two have to cover the rest of the curve: then no root
+        // outside is empty, whatever other vertices the cell has or lacks. (Half the form over rho is the
+        // depth of a conflict, which the rounding of lengths hides up to 4e-7 of rho: it has to be above
+        // that half the balls' margin away, where x and w have moved by 1 + |B| of rho's change and by s's.)
+        // Single precision does, by margins far above its rounding.
+        const float4 fi = to_float( si );
+        const float3 fB = to_float( B ), fn = to_float( n ), fA = f3( fi ) + to_float( A );
+        const float  fal = float( alpha ), fbe = float( beta ), wide = fmaxf( 2.f, 2.f - fal );
+        const float  frc = float( rc ), arf = float( ar ), fas = float( as );
+        float2       g[ 2 ]; // gradient of the third site's form, times -1/2
+        float        r[ 2 ]; // and its radius
+        bool         ahead0 = false, ahead1 = false;
+        float        far = FLT_MAX;
+        const float  root = sqrtf( fmaxf( fal, 0.f ) );
+#pragma unroll 1
+        for ( int a = 0; a < 2; a++ )
+        {
+            const float4 m    = neighbour( c, a ? ends.m[ 1 ] : ends.m[ 0 ] );
+            const float3 em   = f3( m ) - f3( fi );
+            const float2 t    = a ? make_float2( float( along1.x ), float( along1.y ) ) : make_float2( float( along0.x ), float( along0.y ) );
+            const float2 x    = a ? make_float2( float( rho1 ), float( s1 ) ) : make_float2( float( rho0 ), float( s0 ) );
+            const float2 f    = make_float2( fdot( em, fB ) + ( m.w - fi.w ), fdot( em, fn ) );
+            const float  rise = f.x * t.x + f.y * t.y; // the conflict's, along the curve
+            const float  hide = 4e-7f * x.x * x.x * ( wide * fabsf( t.x ) + fabsf( t.y ) ), reach_w = 5e-3f * fmaxf( x.x - fi.w, 0.f ) + 5e-4f;
+            const float  blur = 1e-6f * ( fabsf( fi.x ) + fabsf( fi.y ) + fabsf( fi.z ) + fabsf( m.x ) + fabsf( m.y ) + fabsf( m.z ) );
+            if ( !( fabsf( rise ) > 1e-3f * ( fabsf( f.x * t.x ) + fabsf( f.y * t.y ) ) + blur * ( wide * fabsf( t.x ) + fabsf( t.y ) )
+                    && fabsf( rise ) * reach_w > hide ) )
+                return false;
+            ( a ? ahead1 : ahead0 ) = rise > 0.f;
+            ( a ? g[ 1 ] : g[ 0 ] ) = f;
+            ( a ? r[ 1 ] : r[ 0 ] ) = m.w;
+            if ( fal <= 0.f )
+                continue;
+            // Along s the form is concave where it falls with rho, and then falls on as at the end; else it is
+            // convex, and falls less and less, down to its asymptote's slope. By `slope` or more either way:
+            // a root that passes all the same has a rho of slope sqrt(alpha) / 4e-7 and more.
+            // (The form is that of a conflict only where w is not below -r; w is least where s is 0.)
+            const float out   = rise > 0.f ? 1.f : -1.f;
+            const float least = out * x.y >= 0.f ? x.x - fi.w : ( fbe + sqrtf( fmaxf( fbe * fbe + fal * float( gamma ), 0.f ) ) ) / fal - fi.w;
+            if ( !( least + m.w >= blur ) )
+                return false;
+            const float slope = f.x > 0.f ? out * ( f.x * t.x / t.y + f.y ) : f.x / root + out * f.y;
+            if ( slope > 1e-3f * ( fabsf( f.x ) + fabsf( f.y ) ) + blur * wide && slope * t.y * reach_w > hide )
+            {
+                far = fminf( far, slope * root );
+                continue;
+            }
+            // it ends at the site's other root: another neighbour has to take over there
+            const float q = f.y / f.x, w = 1.f - fal * q * q;
+            const float s = -2.f * q * ( fal * ( x.x + q * x.y ) - fbe ) / w - x.y, rho = x.x + q * ( x.y - s );
+            if ( !( f.x < 0.f && w > 1e-3f && out * ( s - x.y ) > 0.f && fal * rho > fbe && rho < float( kFarRoot ) ) )
+                return false;
+            open.add( a, fA + fB * rho + fn * s, rho - fi.w, fB + fn * ( out * root ), 0.f, least );
+        }
+        // outward of one end is inward of the other
+        if ( ahead0 == ahead1 || !( fabs( ahead ) < near || ahead > 0.0 == ahead1 ) )
+            return false;
+        if ( fal > 0.f )
+            reach.far = fminf( kFarOut * far, float( kFarRoot ) );
+        else
+        {
+            // Half-way round, opposite the piece, each of the two has to hold, or another neighbour has to take
+            // over where it ends, at its other root: the end's mirror image in the gradient (all in the
+            // ellipse's unit circle)
+            const float  low = frc - arf - fi.w;
+            const float2 e0 = make_float2( float( c0.x ), float( c0.y ) ), e1 = make_float2( float( c1.x ), float( c1.y ) );
+            const float  scale = -rsqrtf( 2.f + 2.f * ( e0.x * e1.x + e0.y * e1.y ) );
+            const float2 half  = make_float2( scale * ( e0.x + e1.x ), scale * ( e0.y + e1.y ) );
+            const float  deep  = 8e-7f * ( frc + arf ) * ( frc + arf ) + 2e-6f * ( fabsf( fi.x ) + fabsf( fi.y ) + fabsf( fi.z ) + frc + arf ) * ( arf + fas );
+            if ( !( low + fminf( r[ 0 ], r[ 1 ] ) >= 1e-5f * ( frc + arf ) ) )
+                return false;
+#pragma unroll 1
+            for ( int a = 0; a < 2; a++ )
+            {
+                const float2 f = a ? g[ 1 ] : g[ 0 ], x = a ? e1 : e0;
+                const float2 v = make_float2( f.x * arf, f.y * fas );
+                if ( v.x * ( half.x - x.x ) + v.y * ( half.y - x.y ) > deep )
+                    continue;
+                const float  m = 2.f * ( v.x * x.x + v.y * x.y ) / ( v.x * v.x + v.y * v.y );
+                const float2 y = make_float2( m * v.x - x.x, m * v.y - x.y );
+                open.add( a, fA + fB * ( frc + arf * y.x ) + fn * ( fas * y.y ), frc + arf * y.x - fi.w,
+                          fA + fB * ( frc + arf * half.x ) + fn * ( fas * half.y ), frc + arf * half.x - fi.w, low );
+            }
+        }
         const double3 uT = A + B * rhoT + n * sT;
         const double  wT = rhoT - si.w;
-        reach.ball[ 0 ]  = reach_ball( d3( ends.v[ 0 ] ), rho0 - si.w );
-        reach.ball[ 1 ]  = reach_ball( d3( ends.v[ 1 ] ), rho1 - si.w );
+        reach.ball[ 0 ]  = reach_ball( d3( ends.v[ 0 ] ), fabs( rho0 - si.w ) );
+        reach.ball[ 1 ]  = reach_ball( d3( ends.v[ 1 ] ), fabs( rho1 - si.w ) );
         reach.ball[ 2 ]  = reach_ball( o + uT, sqrt( wT * wT + fmax( 0.0, ddot( uT, uT ) - rhoT * rhoT ) ) );
         return true;
     }
 
+    __device__ __forceinline__ float3 shfl3( float3 v, uint32_t src )
+    {
+        return make_float3( __shfl_sync( 0xffffffffu, v.x, src ), __shfl_sync( 0xffffffffu, v.y, src ), __shfl_sync( 0xffffffffu, v.z, src ) );
+    }
+    __device__ __forceinline__ float4 shfl4f( float4 v, uint32_t src )
+    {
+        return make_float4( __shfl_sync( 0xffffffffu, v.x, src ), __shfl_sync( 0xffffffffu, v.y, src ), __shfl_sync( 0xffffffffu, v.z, src ),
+                            __shfl_sync( 0xffffffffu, v.w, src ) );
+    }
+
+    // Does neighbour m close an open end? It conflicts at the point, not at the end, and where the curve goes on to
+    // (at infinity it stands out by `out`): then all the way. (On a hyperbola its form, see arc_reach, is
+    // concave, and lower at the point than at the end, or convex; on an ellipse it is below 0 on one piece,
+    // which is not the one with the end.) In single precision, by margins of a hundred times its rounding.
+    __device__ __forceinline__ bool closes( float4 at, float4 end, float4 away, float low, bool ellipse, float4 fi, float4 m, float & out )
+    {
+        const float  size = fabsf( fi.x ) + fabsf( fi.y ) + fabsf( fi.z ) + fabsf( m.x ) + fabsf( m.y ) + fabsf( m.z ) + 4.f * fabsf( m.w );
+        const float3 da = f3( m ) - f3( at ), de = f3( m ) - f3( end ), dy = f3( m ) - f3( away );
+        const float  ra = at.w + m.w - 1e-5f * ( size + fabsf( at.w ) ), re = end.w + m.w, ry = away.w + m.w - 1e-5f * ( size + fabsf( away.w ) );
+        out             = fdot( f3( m ) - f3( fi ), f3( away ) ) + m.w - fi.w;
+        return ra > 0.f && fdot( da, da ) < ra * ra && fdot( de, de ) >= re * re && low + m.w >= 0.f
+               && ( ellipse ? ry > 0.f && fdot( dy, dy ) < ry * ry : out > 1e-5f * size );
+    }
+
+    // The open ends that other neighbours close. One lane's edge.
+    __device__ __forceinline__ void close_ends( const CellContext & c, double4 si, uint32_t k, uint32_t l, const ArcEnds & ends,
+                                                const SiteSequence & sites, OpenEnds & open, EdgeReach & reach )
+    {
+        const float4 fi      = to_float( si );
+        const bool   ellipse = reach.kind == kReachArc;
+        for ( uint32_t q = 0; q < sites.count && open.mask; q++ )
+        {
+            const uint32_t u = sites[ q ];
+            if ( u == k || u == l )
+                continue;
+            const float4 m = neighbour( c, u );
+#pragma unroll 1
+            for ( int a = 0; a < 2; a++ )
+            {
+                float out;
+                if ( ( ( open.mask >> a ) & 1u )
+                     && closes( a ? open.at[ 1 ] : open.at[ 0 ], to_float( a ? ends.v[ 1 ] : ends.v[ 0 ] ), a ? open.away[ 1 ] : open.away[ 0 ],
+                                a ? open.low[ 1 ] : open.low[ 0 ], ellipse, fi, m, out ) )
+                {
+                    open.mask &= ~( 1u << a );
+                    reach.far = ellipse ? 0.f : fminf( reach.far, kFarOut * out );
+                }
+            }
+        }
+    }
+
+    // The same for the edges of one cell, one per lane, by the warp: a neighbour per lane.
+    __device__ __forceinline__ void close_ends_together( const CellContext & c, double4 si, uint32_t k, uint32_t l, const ArcEnds & ends,
+                                                         const SiteSequence & sites, OpenEnds & open, EdgeReach & reach )
+    {
+        constexpr uint32_t all = 0xffffffffu;
+        const uint32_t lane = threadIdx.x & 31;
+        const float4   fi   = to_float( si );
+        for ( uint32_t base = 0; base < sites.count; base += 32 )
+        {
+            uint32_t todo = __ballot_sync( all, open.mask != 0 );
+            if ( todo == 0 )
+                break;
+            const bool     has = base + lane < sites.count;
+            const uint32_t u   = has ? sites[ base + lane ] : kNone;
+            const float4   m   = has ? neighbour( c, u ) : make_float4( 0, 0, 0, 0 );
+            while ( todo )
+            {
+                const uint32_t src = __ffs( todo ) - 1;
+                todo &= todo - 1;
+                const uint32_t mask    = __shfl_sync( all, open.mask, src );
+                const uint32_t sk      = __shfl_sync( all, k, src ), sl = __shfl_sync( all, l, src );
+                const bool     ellipse = __shfl_sync( all, reach.kind, src ) == kReachArc;
+#pragma unroll 1
+                for ( int a = 0; a < 2; a++ )
+                {
+                    if ( !( ( mask >> a ) & 1u ) )
+                        continue;
+                    const float4   at   = shfl4f( a ? open.at[ 1 ] : open.at[ 0 ], src ), away = shfl4f( a ? open.away[ 1 ] : open.away[ 0 ], src );
+                    const float4   end  = shfl4f( to_float( a ? ends.v[ 1 ] : ends.v[ 0 ] ), src );
+                    const float    low  = __shfl_sync( all, a ? open.low[ 1 ] : open.low[ 0 ], src );
+                    float          out  = 0.f;
+                    const uint32_t hits = __ballot_sync( all, closes( at, end, away, low, ellipse, fi, m, out ) && has && u != sk && u != sl );
+                    out                 = __shfl_sync( all, out, hits ? __ffs( hits ) - 1 : 0 );
+                    if ( lane == src && hits )
+                    {
+                        open.mask &= ~( 1u << a );
+                        reach.far = ellipse ? 0.f : fminf( reach.far, kFarOut * out );
+                    }
+                }
+            }
+        }
+    }
+
     // Reach of edge (k, l) of cell i: wmax is the largest radius on its arc, `around` the reference's
-    // bounding sphere of the trisector.
+    // bounding sphere of the trisector (`known`: the third sites of the ends are neighbours). To be settled.
     __device__ __forceinline__ EdgeReach edge_reach( const CellContext & c, double4 si, double4 sk, double4 sl, bool hyperbola,
-                                                     const ArcEnds & ends, double wmax, float4 around )
+                                                     const ArcEnds & ends, bool known, double wmax, float4 around, OpenEnds & open )
     {
         EdgeReach    reach;
         const double rmin = c.scene->rmin;
@@ -493,18 +719,29 @@ namespace apo2
         if ( around.w + margin < reach.limit.w )
             reach.limit = make_float4( around.x, around.y, around.z, around.w + margin );
         reach.limit.w += float( c.scene->rmax - rmin ) + low;
-        // a root of radius w touches the plane to L^2 / 2w at a distance of L, at most 2.5 times the
-        // limit's radius
         reach.margin    = 1e-5f * ( reach.limit.w + fabsf( reach.limit.x ) + fabsf( reach.limit.y ) + fabsf( reach.limit.z ) );
-        reach.slab[ 0 ] = reach.slab[ 1 ] = float( 3.2 / kFarRoot ) * reach.limit.w * reach.limit.w + reach.margin;
         reach.diameter  = 2.f * fmaxf( 0.f, float( rmin ) );
         reach.below     = hyperbola && rmin >= 0.0;
-        if ( ends.count == 2 && rmin >= 0.0 && arc_reach( c, si, sk, sl, ends, reach )
-             && ( hyperbola || reach.kind == kReachArc ) )
-            return reach;
-        reach.kind      = kReachBall;
-        reach.ball[ 0 ] = reach.ball[ 1 ] = reach.ball[ 2 ] = reach.limit;
+        if ( !( ends.count == 2 && known && rmin >= 0.0 && arc_reach( c, si, sk, sl, ends, open, reach )
+                && ( hyperbola || reach.kind == kReachArc ) ) )
+        {
+            reach.kind = kReachBall;
+            open.mask  = 0;
+        }
         return reach;
+    }
+    // Once its open ends have been looked at: an arc with one left is searched in the ball.
+    __device__ __forceinline__ void settle( EdgeReach & reach, const OpenEnds & open )
+    {
+        if ( reach.kind == kReachBall || open.mask )
+        {
+            reach.kind      = kReachBall;
+            reach.ball[ 0 ] = reach.ball[ 1 ] = reach.ball[ 2 ] = reach.limit;
+            reach.far       = 1.f;
+        }
+        // a root of radius w touches the plane to L^2 / 2w at a distance of L, at most 2.5 times the
+        // limit's radius
+        reach.slab[ 0 ] = reach.slab[ 1 ] = 3.2f / reach.far * reach.limit.w * reach.limit.w + reach.margin;
     }
 
     // An apex (trisector root in the plane of the centres) counts unless a neighbour other

@@ -239,29 +239,43 @@ namespace apo2
         return lt_eps( flength( f3( to_float( s.si ) ) - f3( s.bsph ) ), known - s.bsph.w );
     }
 
-    // Reach of the search of a bounded edge: the arc's ends and its largest radius.
-    __device__ __forceinline__ void reach_edge( const CellContext & c, EdgeSearch & s, bool ellipse, double4 ev0, double4 ev1 )
+    // Reach of the search of a bounded edge, from the arc's ends and its largest radius. To be settled.
+    __device__ __forceinline__ void reach_edge( const CellContext & c, EdgeSearch & s, bool ellipse, double4 ev0, double4 ev1, ArcEnds & ends,
+                                                OpenEnds & open )
     {
-        const float4 fsi = to_float( s.si );
-        ArcEnds ends;
-        double  wmax = stored_ends( c, s.i, s.si, s.k, s.l, ends, s.hint );
+        double wmax = stored_ends( c, s.i, s.si, s.k, s.l, ends, s.hint );
         if ( ellipse || s.closed )
         {
-            const double4 apex[ 2 ] = { ev0, ev1 };
+#pragma unroll 1
             for ( uint32_t a = 0; a < 2; a++ )
             {
-                bool out = false;
+                const double4 apex = a ? ev1 : ev0;
+                bool          out  = false;
                 for ( uint32_t q = 0; q < s.nbr_count && !out; q++ )
                 {
                     const uint32_t u = s.nbr[ q ];
                     if ( u != s.k && u != s.l )
-                        out = clearly_outside( c.sites[ u ], apex[ a ] );
+                        out = clearly_outside( c.sites[ u ], apex );
                 }
                 if ( !out )
-                    wmax = fmax( wmax, apex[ a ].w );
+                    wmax = fmax( wmax, apex.w );
             }
         }
-        s.reach = edge_reach( c, s.si, s.sk, s.sl, s.hyperbola, ends, wmax, s.bsph );
+        // only neighbours bound the arc, are tested first, and skipped by the walk
+        for ( uint32_t h = 0; h < 2; h++ )
+            if ( s.hint[ h ] != kNone && !in_sorted( s.nbr, s.nbr_count, s.hint[ h ] ) )
+                s.hint[ h ] = kNone;
+        const auto known = [ & ]( uint32_t m ) { return m == s.hint[ 0 ] || m == s.hint[ 1 ]; };
+        s.reach = edge_reach( c, s.si, s.sk, s.sl, s.hyperbola, ends, ends.count == 2 && known( ends.m[ 0 ] ) && known( ends.m[ 1 ] ), wmax,
+                              s.bsph, open );
+        s.covered = wmax <= 1.001 * double( c.largest[ s.i ] );
+    }
+
+    // The reach once its open ends have been looked at, and the planes that need not be.
+    __device__ __forceinline__ void settle_edge( const CellContext & c, EdgeSearch & s, const OpenEnds & open )
+    {
+        const float4 fsi = to_float( s.si );
+        settle( s.reach, open );
         if ( s.reach.kind == kReachArcPlanes )
         {
             bool open1 = true, open2 = true;
@@ -271,8 +285,8 @@ namespace apo2
                 if ( u == s.k || u == s.l || u >= c.n )
                     continue;
                 const float4 m = c.sites_f[ u ];
-                open1          = open1 && !far_roots_blocked( s.planes.n1, fsi, m );
-                open2          = open2 && !far_roots_blocked( s.planes.n2, fsi, m );
+                open1          = open1 && !far_roots_blocked( s.planes.n1, fsi, m, s.reach.far );
+                open2          = open2 && !far_roots_blocked( s.planes.n2, fsi, m, s.reach.far );
             }
             if ( !open1 )
                 s.reach.slab[ 0 ] = -FLT_MAX;
@@ -282,12 +296,16 @@ namespace apo2
                 s.reach.kind = kReachArc;
         }
         const uint2 around = c.around[ s.i ];
-        s.covered          = wmax <= 1.001 * double( c.largest[ s.i ] );
         s.from             = s.covered ? ( s.reach.kind == kReachArc ? around.x : around.y ) : 0u;
-        // only neighbours are tested first, and skipped by the walk
-        for ( uint32_t h = 0; h < 2; h++ )
-            if ( s.hint[ h ] != kNone && !in_sorted( s.nbr, s.nbr_count, s.hint[ h ] ) )
-                s.hint[ h ] = kNone;
+    }
+    __device__ __forceinline__ SiteSequence neighbours( const EdgeSearch & s ) { return { s.nbr, s.nbr_count, 0u }; }
+    __device__ __forceinline__ void set_reach( const CellContext & c, EdgeSearch & s, bool ellipse, double4 ev0, double4 ev1 )
+    {
+        ArcEnds  ends;
+        OpenEnds open;
+        reach_edge( c, s, ellipse, ev0, ev1, ends, open );
+        close_ends( c, s.si, s.k, s.l, ends, neighbours( s ), open, s.reach );
+        settle_edge( c, s, open );
     }
 
     // The walk is bound by the node steps (two boxes against three balls and two planes, 50 to 90
@@ -344,19 +362,25 @@ namespace apo2
         // A root is empty when no neighbour other than k, l conflicts with it: the neighbours
         // bounding the edge's arc go first (a root outside the arc is nearly always inside one of
         // them), then the whole sorted list. The conjunction is the same.
+        const auto conflicts = [ & ]( uint32_t u, double4 root ) {
+            return c.fp32 ? site_conflict<true>( c, u, root, untallied ) : site_conflict<false>( c, u, root, untallied );
+        };
+#pragma unroll 1
         for ( uint32_t r = 0; r < 2; r++ )
         {
-            bool ok = true;
+            const double4 root = r ? x[ 1 ] : x[ 0 ];
+            bool          ok   = true;
+#pragma unroll 1
             for ( uint32_t h = 0; h < 2 && ok; h++ )
-                if ( s.hint[ h ] != kNone )
-                    ok = !( c.fp32 ? site_conflict<true>( c, s.hint[ h ], x[ r ], untallied )
-                                   : site_conflict<false>( c, s.hint[ h ], x[ r ], untallied ) );
+            {
+                const uint32_t u = h ? s.hint[ 1 ] : s.hint[ 0 ];
+                ok               = u == kNone || !conflicts( u, root );
+            }
             for ( uint32_t q = 0; q < s.nbr_count && ok; q++ )
             {
                 const uint32_t u = s.nbr[ q ];
                 if ( u != s.k && u != s.l )
-                    ok = !( c.fp32 ? site_conflict<true>( c, u, x[ r ], untallied )
-                                   : site_conflict<false>( c, u, x[ r ], untallied ) );
+                    ok = !conflicts( u, root );
             }
             if ( ok )
                 return true;
@@ -371,9 +395,9 @@ namespace apo2
         atomicOr( &b.cell_flag[ t ], kFlagFound );
     }
 
-    // Edge e of task t, ready for the search; false if it needs none.
+    // Edge e of task t, bounded; false if it needs no search.
     __device__ __forceinline__ bool load_edge( const CellContext & c, const uint32_t * tasks, const SpecBuffers & b, uint32_t t,
-                                               uint32_t e, EdgeSearch & s )
+                                               uint32_t e, EdgeSearch & s, bool & ellipse, double4 & ev0, double4 & ev1 )
     {
         s.t           = t;
         s.e           = e;
@@ -390,12 +414,8 @@ namespace apo2
             return false;
         s.sk = c.sites[ s.k ];
         s.sl = c.sites[ s.l ];
-        double4    ev0, ev1;
-        const bool ellipse = bound_edge( s, ev0, ev1 );
-        if ( covers_edge( s, c.known_radii[ s.i ] ) )
-            return false;
-        reach_edge( c, s, ellipse, ev0, ev1 );
-        return true;
+        ellipse = bound_edge( s, ev0, ev1 );
+        return !covers_edge( s, c.known_radii[ s.i ] );
     }
 
     // Edges of cells with few surroundings, nearly all: a warp per cell collects the sites, other than
@@ -430,7 +450,8 @@ namespace apo2
                 continue;
             const uint32_t * nbr   = b.nbr + size_t( t ) * kNbrCap;
             const uint32_t   known = b.nbr_count[ t ];
-            float4           ball  = touch_ball( c, c.sites[ i ], c.largest[ i ] );
+            const double4    si    = c.sites[ i ];
+            float4           ball  = touch_ball( c, si, c.largest[ i ] );
             ball.w += 1.001f * float( c.scene->rmax - c.scene->rmin );
             // far more than the list holds, at the scene's mean density: not worth collecting
             if ( 4.2f * ball.w * ball.w * ball.w * density > 4.f * float( kListCap ) )
@@ -442,7 +463,17 @@ namespace apo2
             for ( uint32_t base = 0; base < edges; base += 32 )
             {
                 EdgeSearch s;
-                bool       open = base + lane < edges && load_edge( c, tasks, b, t, base + lane, s );
+                ArcEnds    ends;
+                OpenEnds   loose;
+                bool       ellipse;
+                double4    ev0, ev1;
+                bool       open = base + lane < edges && load_edge( c, tasks, b, t, base + lane, s, ellipse, ev0, ev1 );
+                if ( open )
+                    reach_edge( c, s, ellipse, ev0, ev1, ends, loose );
+                __syncwarp();
+                close_ends_together( c, si, s.k, s.l, ends, SiteSequence { nbr, known, 0u }, loose, s.reach );
+                if ( open )
+                    settle( s.reach, loose );
                 if ( open && !s.covered )
                 {
                     const uint32_t slot = atomicAdd( b.heavy_count, 1u );
@@ -452,15 +483,26 @@ namespace apo2
                         send_to_exact( b, s.t, s.e );
                     open = false;
                 }
-                for ( uint32_t q = 0; q < listed; q++ )
+                // 32 sites at a time: first which of them are near, a bit each, then every lane its own
+                for ( uint32_t first = 0; first < listed; first += 32 )
                 {
-                    const bool near = open && within( s.reach, s.planes, list[ q ] );
-                    if ( !__any_sync( 0xffffffffu, near ) )
-                        continue;
-                    if ( near && contributes( c, s, ids[ q ] ) )
+                    const uint32_t block = min( listed - first, 32u );
+                    uint32_t       near  = 0;
+                    for ( uint32_t q = 0; q < block; q++ )
+                        near |= uint32_t( within<false>( s.reach, s.planes, list[ first + q ] ) ) << q;
+                    near = open ? near : 0u;
+                    while ( __any_sync( 0xffffffffu, near != 0 ) )
                     {
-                        send_to_exact( b, s.t, s.e );
-                        open = false;
+                        if ( near == 0 )
+                            continue;
+                        const uint32_t q = __ffs( near ) - 1;
+                        near &= near - 1;
+                        if ( contributes( c, s, ids[ first + q ] ) )
+                        {
+                            send_to_exact( b, s.t, s.e );
+                            open = false;
+                            near = 0;
+                        }
                     }
                 }
             }
@@ -520,6 +562,8 @@ namespace apo2
                             else
                                 hi = mid;
                         }
+                        bool             ellipse;
+                        double4          ev0, ev1;
                         s.t              = lo;
                         const uint32_t e = uint32_t( item - b.item_offset[ s.t ] );
                         s.e              = e;
@@ -528,8 +572,9 @@ namespace apo2
                             // no neighbour list for this cell: the exact path searches this edge
                             atomicOr( &b.maybe_bits[ size_t( s.t ) * kMaybeWords + ( e >> 5 ) ], 1u << ( e & 31 ) );
                         }
-                        else if ( load_edge( c, tasks, b, lo, e, s ) )
+                        else if ( load_edge( c, tasks, b, lo, e, s, ellipse, ev0, ev1 ) )
                         {
+                            set_reach( c, s, ellipse, ev0, ev1 );
                             active = true;
                             sp     = 0;
                             node   = s.from;
@@ -695,7 +740,7 @@ namespace apo2
         s.nbr_count   = b.nbr_count[ s.t ];
         double4    ev0, ev1;
         const bool ellipse = bound_edge( s, ev0, ev1 );
-        reach_edge( c, s, ellipse, ev0, ev1 );
+        set_reach( c, s, ellipse, ev0, ev1 );
     }
 
     __global__ void __launch_bounds__( kHeavyBlock, 4 ) k_edge_heavy( CellContext c, const uint32_t * __restrict__ tasks,
