@@ -420,7 +420,7 @@ namespace
         total += align256( 4 * size_t( n ) ) * 2 + align256( 4 * scanWords * 2 ) + align256( 16 );
         total += align256( spec_bytes( n ) );
         total += align256( walk_scratch_bytes( n ) ) + align256( 4 );
-        total += align256( 4 * size_t( n ) ) + align256( 8 * size_t( n ) );
+        total += align256( 4 * size_t( n ) ) * 2;
         return total;
     }
 
@@ -490,7 +490,7 @@ namespace
         c.deferred        = h->spec.exact_tasks; // not in use while the cell passes run
         c.deferred_count  = h->spec.exact_count;
         c.largest         = a.take<float>( n );
-        c.around          = a.take<uint2>( n );
+        c.around          = a.take<uint32_t>( n );
         c.fp32            = opt.precision == APO2_PRECISION_FP32_FILTER ? 1u : 0u;
         c.codes           = t.codes;
         sort_scratch_carve( h->sort, sortBase, n, h->error );

@@ -1469,9 +1469,7 @@ namespace apo2
             // for the edge searches
             const double last  = largest_radius( w );
             const float4 touch = touch_ball( c, si, last );
-            uint2        around;
-            around.y = node_around( c.nodes, n, make_float4( touch.x, touch.y, touch.z, touch.w + 1.001f * float( c.scene->rmax - c.scene->rmin ) ) );
-            around.x = node_around( c.nodes, n, touch, around.y );
+            const uint32_t around = node_around( c.nodes, n, make_float4( touch.x, touch.y, touch.z, touch.w + 1.001f * float( c.scene->rmax - c.scene->rmin ) ) );
             if ( lane == 0 )
             {
                 c.largest[ i ] = float( last );
@@ -1969,6 +1967,8 @@ namespace apo2
                     for ( int q = 0; q < 2; q++ )
                         p.reach.slab[ q ] = __shfl_sync( kFull, reach.slab[ q ], src );
                     p.reach.limit = shfl4f( reach.limit, src );
+                    p.reach.flat  = shfl4f( reach.flat, src );
+                    p.reach.near  = __shfl_sync( kFull, reach.near, src );
                     p.reach.kind  = __shfl_sync( kFull, reach.kind, src );
                     p.reach.diameter = __shfl_sync( kFull, reach.diameter, src );
                     p.reach.margin   = __shfl_sync( kFull, reach.margin, src );

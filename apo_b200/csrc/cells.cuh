@@ -83,10 +83,9 @@ namespace apo2
         uint32_t *       deferred       = nullptr; // cells that outgrew the small slots, and their number
         uint32_t *       deferred_count = nullptr;
         // left by the vertex validation for the edge searches of the same round: the largest vertex
-        // radius of each cell, and the nodes around everything that its spheres can touch (x) and
-        // around everything within the general bound of its edges (y)
+        // radius of each cell, and the node around everything within the general bound of its edges
         float * largest = nullptr;
-        uint2 * around  = nullptr;
+        uint32_t * around = nullptr;
         // learned k-proposal (null: the plain form): the network, the Morton codes its features
         // read, and the proposed rank of every site (written by the first kNN step)
         const ProposalNet * proposal   = nullptr;
@@ -225,7 +224,7 @@ namespace apo2
     // duplicate sites, and where roots went lost to rounding, a cell lacks some, and an arc between two
     // of the others is not all that is open.
     //
-    // One kind of contributor lies outside the balls all the same.
+    // Two kinds of contributor lie outside the balls all the same.
     //
     // A root so far away that the single-precision lengths of the emptiness test cannot tell the
     // neighbours apart (its radius was 7e7 and more where it happened, once in some ten builds, on edges
@@ -235,16 +234,26 @@ namespace apo2
     // plane, so on a hyperbolic trisector the boxes that reach one of the two planes within the general
     // bound are entered too (kReachArcPlanes); an elliptic one has no point further than its apex. Most
     // planes are out, though (far_roots_blocked).
+    //
+    // A root of four sites whose centres lie in a plane, but for rounding: its height over the plane is a quotient
+    // of two small numbers, and it can come out anywhere. Of relative errors of 1.1e-16 in coordinates of
+    // size L and a height h of c_j over the plane of the other three, the root's height is off by up to
+    // 1e-8 L sqrt(w d) / h, d the difference of the radii, which is inside the balls' margin from h = 1.7e-6 L
+    // sqrt(d) on; centres nearer than kFlat L_1 (L_1 the sum over the axes, and 1 / sin of the triangle's angle
+    // more) are tested within the general bound.
     // ---------------------------------------------------------------------------------
     constexpr uint32_t kReachBall = 0, kReachArc = 1, kReachArcPlanes = 2;
     constexpr double   kFarRoot   = 2.5e5; // radius from which a root counts as far: single precision is off by 0.1 there
     constexpr float    kFarOut    = 2.5e6f; // ... by 4e-7 of the radius: least radius, by the depth of the conflict
+    constexpr float    kFlat      = 2e-6f; // of the coordinates: centres so near to a plane count as in it
 
     struct EdgeReach
     {
         float4   ball[ 3 ]; // kReachBall: the same one three times
         float4   limit;     // ball holding every site that the planes let in
         float    slab[ 2 ]; // kReachArcPlanes: how near to each tangent plane it has to come
+        float4   flat;      // the plane of the three centres (normal, offset), and how near a centre
+        float    near;      // has to come to it
         // hyperbolic trisectors: a contributor lies wholly below both planes (algorithm.inl:695-700), so
         // a box has to go below them by a smallest sphere's diameter; less this rounding margin
         float    diameter, margin;
@@ -289,13 +298,20 @@ namespace apo2
         const float  r = fmaxf( fmaxf( b.hi.x - b.lo.x, b.hi.y - b.lo.y ), b.hi.z - b.lo.z ) * .5f;
         return make_float4( m.x, m.y, m.z, r + 1e-6f * ( fabsf( m.x ) + fabsf( m.y ) + fabsf( m.z ) + fabsf( r ) ) );
     }
+    // Distance of a centre from the plane (at least so much for the centres in a box).
+    __device__ __forceinline__ float off_plane( float4 p, const Box & b )
+    {
+        const float3 n = f3( p ), m = ( b.lo + b.hi ) * .5f, h = ( b.hi - b.lo ) * .5f;
+        return fabsf( fdot( n, m ) - p.w ) - ( fabsf( n.x ) * h.x + fabsf( n.y ) * h.y + fabsf( n.z ) * h.z );
+    }
+    __device__ __forceinline__ float off_plane( float4 p, float4 site ) { return fabsf( fdot( f3( p ), f3( site ) ) - p.w ); }
     // May box or site `x` be, or hold, a contributor? The balls are tested without branches: a walk's
     // lanes would take them all the same.
     template<bool Limited = true, class X>
     __device__ __forceinline__ bool within( const EdgeReach & a, const TangentPlanes & t, const X & x )
     {
         bool in   = meets( a.ball[ 0 ], x ) | meets( a.ball[ 1 ], x ) | meets( a.ball[ 2 ], x );
-        bool more = false;
+        bool more = off_plane( a.flat, x ) <= a.near;
         if ( a.below )
         {
             const float2 h1 = heights( t.n1, t.p1, a.diameter, x ), h2 = heights( t.n2, t.p2, a.diameter, x );
@@ -603,6 +619,11 @@ namespace apo2
                           fA + fB * ( frc + arf * half.x ) + fn * ( fas * half.y ), frc + arf * half.x - fi.w, low );
             }
         }
+        // how near to the plane of the centres a root is not to be trusted
+        const float size = float( fmax( fabs( c.scene->lo[ 0 ] ), fabs( c.scene->hi[ 0 ] ) ) + fmax( fabs( c.scene->lo[ 1 ] ), fabs( c.scene->hi[ 1 ] ) )
+                                  + fmax( fabs( c.scene->lo[ 2 ] ), fabs( c.scene->hi[ 2 ] ) ) );
+        reach.flat       = make_float4( float( n.x ), float( n.y ), float( n.z ), float( ddot( n, o ) ) );
+        reach.near       = kFlat * size * sqrtf( float( gkk * gll * inv ) );
         const double3 uT = A + B * rhoT + n * sT;
         const double  wT = rhoT - si.w;
         reach.ball[ 0 ]  = reach_ball( d3( ends.v[ 0 ] ), fabs( rho0 - si.w ) );
@@ -737,6 +758,8 @@ namespace apo2
         {
             reach.kind      = kReachBall;
             reach.ball[ 0 ] = reach.ball[ 1 ] = reach.ball[ 2 ] = reach.limit;
+            reach.flat      = make_float4( 0.f, 0.f, 0.f, 0.f );
+            reach.near      = -1.f;
             reach.far       = 1.f;
         }
         // a root of radius w touches the plane to L^2 / 2w at a distance of L, at most 2.5 times the
@@ -756,8 +779,9 @@ namespace apo2
 
     // The node every walk inside a ball may start from: from the root down to where both children
     // meet the ball. The walk would go the same way, one box after another, without meeting a leaf.
-    __device__ __forceinline__ uint32_t node_around( const WideNode * nodes, uint32_t n, float4 ball, uint32_t node = 0 )
+    __device__ __forceinline__ uint32_t node_around( const WideNode * nodes, uint32_t n, float4 ball )
     {
+        uint32_t node = 0;
         while ( true )
         {
             Box      lb, rb;

@@ -269,6 +269,7 @@ namespace apo2
         s.reach = edge_reach( c, s.si, s.sk, s.sl, s.hyperbola, ends, ends.count == 2 && known( ends.m[ 0 ] ) && known( ends.m[ 1 ] ), wmax,
                               s.bsph, open );
         s.covered = wmax <= 1.001 * double( c.largest[ s.i ] );
+        s.from    = s.covered ? c.around[ s.i ] : 0u;
     }
 
     // The reach once its open ends have been looked at, and the planes that need not be.
@@ -295,8 +296,6 @@ namespace apo2
             if ( !open1 && !open2 )
                 s.reach.kind = kReachArc;
         }
-        const uint2 around = c.around[ s.i ];
-        s.from             = s.covered ? ( s.reach.kind == kReachArc ? around.x : around.y ) : 0u;
     }
     __device__ __forceinline__ SiteSequence neighbours( const EdgeSearch & s ) { return { s.nbr, s.nbr_count, 0u }; }
     __device__ __forceinline__ void set_reach( const CellContext & c, EdgeSearch & s, bool ellipse, double4 ev0, double4 ev1 )
@@ -456,7 +455,7 @@ namespace apo2
             // far more than the list holds, at the scene's mean density: not worth collecting
             if ( 4.2f * ball.w * ball.w * ball.w * density > 4.f * float( kListCap ) )
                 continue;
-            const uint32_t listed = collect_sites( c, i, ball, c.around[ i ].y, list, ids, ids + kListCap,
+            const uint32_t listed = collect_sites( c, i, ball, c.around[ i ], list, ids, ids + kListCap,
                                                    [ & ]( uint32_t j ) { return in_sorted( nbr, known, j ); } );
             if ( listed == kNone )
                 continue; // its items stay

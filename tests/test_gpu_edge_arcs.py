@@ -3,7 +3,9 @@ compared with those of a build that searched the whole ball around the cell's si
 of its stores below, where they were also the same with the bounding sphere in the ball's place):
 
 - sets with a tenth of the sites twice: a cell lacks vertices that a duplicate neighbour took, so the
-  arc between two of the others is not all of the edge that is open.
+  arc between two of the others is not all of the edge that is open;
+- lattices with a jitter of 1e-4: where four centres lie in a plane but for the rounding of their
+  coordinates, the root that their spheres touch comes out at any height over it.
 """
 import hashlib
 
@@ -50,3 +52,22 @@ def stores(sites, status_ok, precision):
 ])
 def test_duplicate_sites(n, seed, lognormal, status_ok, digest, precision):
     assert stores(duplicates(n, seed, lognormal), status_ok, precision) == digest
+
+
+def layered(side: int, seed: int) -> np.ndarray:
+    rng = np.random.default_rng(seed)
+    x = np.stack(np.meshgrid(*[np.arange(side) * 3.] * 3, indexing="ij"), -1).reshape(-1, 3) + rng.normal(0, 1e-4, (side ** 3, 3))
+    return np.concatenate([x, np.clip(rng.lognormal(0, .5, side ** 3), .2, 3.)[:, None]], axis=1).astype(np.float32)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("side,seed,digest", [
+    (7, 0, "128ba5fe2085b587b6989fb2d969ba3d"),
+    (7, 40, "2e51dd43199e9486b18b26e70061c732"),
+    (8, 0, "9a78d0b7f0eee5fe01194b1661143c72"),
+    (8, 18, "022aec58a6350f12d7dee0f2ca564e47"),
+    (8, 52, "378b1854427f1ff868cc8f522eddcf01"),
+    (8, 55, "b9d92b5d7458a8e79ab8de9a029c1d4e"),
+])
+def test_coplanar_sites(side, seed, digest, precision):
+    assert stores(layered(side, seed), True, precision) == digest
