@@ -1301,7 +1301,8 @@ namespace apo2
             load_cell( c, w, i, si, true, true );
             const float known = c.known_radii[ i ];
             // the walks of the first pass start at the node around everything that the cell's spheres
-            // come near to
+            // come near to; not those of vertices elsewhere (one whose root the solve with sorted sites
+            // does not give has its record, and the origin for a position)
             float4 field = touch_ball( c, si, largest_radius( w ) );
             field.w += 2e-2f + 2e-5f * ( fabsf( field.x ) + fabsf( field.y ) + fabsf( field.z ) + field.w );
             const uint32_t start = node_around( c.nodes, n, field );
@@ -1352,7 +1353,7 @@ namespace apo2
                 {
                     uint2    stack[ kStack ];
                     int      sp         = 0;
-                    uint32_t node       = pass == 0 && 2.f * fmaxf( fc.w, 0.f ) + float( si.w ) + bound <= field.w ? start : 0u;
+                    uint32_t node       = pass == 0 && flength( f3( fc ) - f3( field ) ) + fmaxf( fc.w, 0.f ) + bound <= field.w ? start : 0u;
                     float    best       = pass == 0 ? bound : FLT_MAX;
                     bool     walking    = searching;
                     uint32_t walk_steps = 0;
