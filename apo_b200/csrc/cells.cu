@@ -741,7 +741,7 @@ namespace apo2
     }
 
     // Small slots: has the cell outgrown them (warp-wide)? The caller then leaves it, with the error
-    // flags it had before, to the launch over the deferred cells.
+    // flags and counts it had before, to the launch over the deferred cells.
     template<class W>
     __device__ __forceinline__ bool outgrown( uint32_t err )
     {
@@ -1094,6 +1094,7 @@ namespace apo2
                 continue; // learned form: this cell was proposed within k, so it has one step only
             const double4  si    = c.sites[ i ];
             const uint32_t noted = err, counted = lane_id() < kCounters ? counts[ lane_id() ] : 0u;
+            const FilterTally tallied = w.tally;
             if ( mode == kCellsNext )
             {
                 if ( too_large<W>( c, i ) )
@@ -1162,7 +1163,8 @@ namespace apo2
             }
             if ( outgrown<W>( err ) )
             {
-                err = noted;
+                err     = noted;
+                w.tally = tallied;
                 __syncwarp();
                 if ( lane_id() < kCounters )
                     counts[ lane_id() ] = counted;
@@ -1291,8 +1293,9 @@ namespace apo2
             const uint8_t  status = c.status[ i ];
             if ( status == kFullyValidated || status == kBuried )
                 continue;
-            const double4  si    = c.sites[ i ];
-            const uint32_t noted = err;
+            const double4     si      = c.sites[ i ];
+            const uint32_t    noted   = err;
+            const FilterTally tallied = w.tally;
             if ( too_large<W>( c, i ) )
             {
                 defer_cell( c, i );
@@ -1462,7 +1465,8 @@ namespace apo2
             }
             if ( outgrown<W>( err ) )
             {
-                err = noted;
+                err     = noted;
+                w.tally = tallied;
                 defer_cell( c, i );
                 continue;
             }

@@ -44,3 +44,23 @@ def test_cells_that_outgrow_the_small_slots(around, lo, hi, steps, precision):
     st = algo.stats()
     assert st["error_flags"] == 0
     algo.close()
+
+
+@pytest.mark.parametrize("kind", ["cells", "vertices"])
+def test_filter_counts_without_the_attempts_that_are_done_again(kind):
+    """The FP32 filter's counts of a build that does cells again with the full slots (kNN cells from 4096
+    cells on, vertex validation from 400,000) are those of its shards, which are too small for that."""
+    import apo_b200
+    from apo_b200 import generators
+    sites = clusters(70, 2.0, 2.3) if kind == "cells" else generators.lognormal_cloud(410000, 400.0 * (410000 / 5e6) ** (1 / 3), 3)
+    counts = []
+    for shards in (1, 2):
+        total = [0, 0]
+        for s in range(shards):
+            algo = apo_b200.AlgorithmGPU(sites, knnValidationStep=6 if kind == "cells" else 1, precision="fp32", shard=(s, shards))
+            algo.build()
+            st = algo.stats()
+            total = [total[0] + st["filter_tests"], total[1] + st["filter_escalations"]]
+            algo.close()
+        counts.append(total)
+    assert counts[0] == counts[1] and counts[0][0] > 0
