@@ -1851,7 +1851,7 @@ namespace apo2
                         err |= kErrWalk;
                         walking = false;
                     }
-                    if ( walking && walk_steps > ( proof.maybe_bits ? kLaneWalkLeft : kLaneWalk ) )
+                    if ( walking && walk_steps > ( monotone ? kLaneWalkLeft : kLaneWalk ) )
                     {
                         // a long search: its position (current node, then the stack from the
                         // top) goes to scratch and the warp finishes it below

@@ -164,7 +164,9 @@ namespace apo2
     // one after another by the whole warp: they go there after 4 steps (longest launches of the pass
     // summed over the rounds, 256 -> 32 -> 4 steps: 100,000 uniform sites 5.4 -> 2.6 -> 1.8 ms, 10,000 0.42 ->
     // 0.29 -> 0.26, 300,000 log-normal 3.9 -> 3.7 -> 3.6, 800,000 8.2 -> 8.6 -> 8.2, 1M protein-like 1.1 ->
-    // 0.6 -> 0.6). Without that search every edge walks, 32 at a time, and lanes keep kLaneWalk.
+    // 0.6 -> 0.6). Without that search, and once a neighbour has left the cell and its proofs lapse, every edge
+    // walks, 32 at a time, and lanes keep kLaneWalk (4 steps there too: the longest launch of 5M log-normal
+    // sites 766 and 777 ms, all of the 126^3 lattice 1648 and 1645).
     constexpr uint32_t kLaneWalkLeft     = 4;
 #ifndef APO2_COOP_WIDTH
 #define APO2_COOP_WIDTH 4
