@@ -488,7 +488,6 @@ namespace
         c.walk_scratch    = a.take<uint32_t>( walk_scratch_bytes( n ) / sizeof( uint32_t ) );
         c.work_counter    = a.take<uint32_t>( 1 );
         c.deferred        = h->spec.exact_tasks; // not in use while the cell passes run
-        c.deferred_count  = h->spec.exact_count;
         c.largest         = a.take<float>( n );
         c.around          = a.take<uint32_t>( n );
         c.fp32            = opt.precision == APO2_PRECISION_FP32_FILTER ? 1u : 0u;

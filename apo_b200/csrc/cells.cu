@@ -1051,8 +1051,6 @@ namespace apo2
     {
         extern __shared__ __align__( 16 ) unsigned char smem[];
         const uint32_t warp  = threadIdx.x >> 5;
-        const uint32_t gwarp = blockIdx.x * ( kCellBlock / 32 ) + warp;
-        const uint32_t nwarp = gridDim.x * ( kCellBlock / 32 );
         using W = WarpCell<Fp32, Small>;
         W              w = carve<W>( smem, warp, 0 );
         uint32_t       err   = 0;
@@ -1063,8 +1061,6 @@ namespace apo2
             counts[ lane_id() ] = 0;
         __syncwarp();
         // cells are taken one at a time from a shared counter (uneven cells, see bisector pass)
-        ( void ) gwarp;
-        ( void ) nwarp;
         const uint32_t total = deferred ? *c.deferred_count : c.hi - c.lo;
         while ( true )
         {
@@ -1269,8 +1265,6 @@ namespace apo2
     {
         extern __shared__ __align__( 16 ) unsigned char smem[];
         const uint32_t warp  = threadIdx.x >> 5;
-        const uint32_t gwarp = blockIdx.x * ( kCellBlock / 32 ) + warp;
-        const uint32_t nwarp = gridDim.x * ( kCellBlock / 32 );
         const uint32_t lane  = lane_id();
         using W = WarpCell<Fp32, Small>;
         W              w = carve<W>( smem, warp, 0 );
@@ -1279,8 +1273,6 @@ namespace apo2
         const uint32_t n     = c.n;
         const float    rmax  = float( c.scene->rmax );
         // tasks are taken one at a time from a shared counter (uneven cells, see bisector pass)
-        ( void ) gwarp;
-        ( void ) nwarp;
         while ( true )
         {
             uint32_t t = 0;
@@ -1683,7 +1675,6 @@ namespace apo2
         extern __shared__ __align__( 16 ) unsigned char smem[];
         const uint32_t warp  = threadIdx.x >> 5;
         const uint32_t gwarp = blockIdx.x * ( kCellBlock / 32 ) + warp;
-        const uint32_t nwarp = gridDim.x * ( kCellBlock / 32 );
         const uint32_t lane  = lane_id();
         using W = WarpCell<Fp32>;
         W              w = carve<W>( smem, warp, 0 );
@@ -1693,7 +1684,6 @@ namespace apo2
         uint32_t *     frontier = c.walk_scratch + size_t( gwarp ) * kWalkScratchWords;
         uint32_t *     saved    = frontier + kCoopCap + lane * ( kStack + 1 );
         // tasks are taken one at a time from a shared counter; `gwarp` only names the scratch
-        ( void ) nwarp;
         while ( true )
         {
             uint32_t t = 0;
@@ -2627,16 +2617,13 @@ namespace apo2
         return size_t( cell_grid( cells ) ) * ( kCellBlock / 32 ) * kWalkScratchWords * sizeof( uint32_t );
     }
 
-#ifndef APO2_KNN_WARPS
-#define APO2_KNN_WARPS ( 148u * 32u )
-#endif
     void launch_knn( const CellContext & c, uint32_t step, cudaStream_t s )
     {
         // A warp lasts as long as its lanes' walks together, which part at every node: few sites are
         // spread over more warps, 32 per SM, with down to 4 lanes each (1,000 sites 220 -> 130 us, 10,000
         // 308 -> 208 us, 61,000 429 -> 412 us).
         uint32_t lanes = 4;
-        while ( lanes < 32 && c.n > lanes * APO2_KNN_WARPS )
+        while ( lanes < 32 && c.n > lanes * 148u * 32u )
             lanes *= 2;
         const uint32_t per_block = lanes * ( kKnnBlock / 32 );
         const uint32_t blocks    = ( c.n + per_block - 1 ) / per_block;
@@ -2651,7 +2638,8 @@ namespace apo2
     // log-normal cloud 60.2 -> 57.0, 46^3 lattice 6.03 -> 5.55. In the vertex validation a few hull
     // cells do, and the second launch lasts as long as the longest of them, 4 to 10 ms: 1M protein
     // packing 190.5 -> 160.1 + 5.8 ms, 1M log-normal cloud 107.2 -> 95.0 + 9.9, but 61k protein 13.0 ->
-    // 10.9 + 3.8.
+    // 10.9 + 3.8. In between, both launches: protein 150k 29.5 -> 29.3, 250k 48.3 -> 44.8, 400k 76.4 -> 68.8,
+    // log-normal 150k 19.2 -> 22.7, 250k 29.2 -> 34.0, 400k 44.5 -> 46.5 ms.
     constexpr uint32_t kSmallCellsFrom = 4096, kSmallVerticesFrom = 400000;
 
     static CellContext with_counter( CellContext c, ZeroWords & z )

@@ -180,10 +180,7 @@ namespace apo2
     // lists of up to 64 / 128 / 256 / 384 / 1024 sites (0: 75.5, 105.9 and 7.7 ms): 1M protein packing
     // 76.9 / 73.8 / 72.7 / 74.6 / 88.6 ms, 1M log-normal cloud 112 / 107 / 86 / 83 / 75 ms, 46^3
     // lattice 6.0 / 5.9 / 6.0 / 5.8 / 5.9 ms.
-#ifndef APO2_EDGE_LIST
-#define APO2_EDGE_LIST 384
-#endif
-    constexpr uint32_t kListCap   = APO2_EDGE_LIST;
+    constexpr uint32_t kListCap   = 384;
     constexpr uint32_t kListStack = 4096;
     static_assert( 5 * kListCap + kListStack <= kWalkScratchWords && kWalkScratchWords % 4 == 0, "the list fits the scratch" );
 
@@ -917,7 +914,8 @@ namespace apo2
     // Edge-parallel edge validation with an exact per-cell fallback (speculate.cu).
     struct SpecBuffers
     {
-        uint32_t * nbr          = nullptr; // per task: sorted unique neighbour ids (64 slots)
+        // the counters (item_counter and every *_count and *_next) are null until a launch takes its own
+        uint32_t * nbr          = nullptr; // per task: sorted unique neighbour ids (kNbrCap slots)
         uint32_t * nbr_count    = nullptr;
         uint32_t * item_count   = nullptr; // per task: edges to search; scanned into item_offset
         uint32_t * item_offset  = nullptr;

@@ -292,8 +292,8 @@ namespace apo2
     // Up to a tile of keys: every key's place is the number of keys before it (smaller, or equal and
     // earlier), counted by 16 threads per key over all keys. A pass of the radix sort is 13 us for any
     // number of keys up to a tile, latency of its phases, and there are eight: 100 sites 102 -> 11 us,
-    // 1000 sites 131 -> 19 us (both launches). The counting grows with the square of the keys, so larger
-    // sets keep the radix sort.
+    // 1000 sites 138 -> 17 us, 2000 139 -> 21, 3000 144 -> 25, 4096 144 -> 30 (both launches). Larger sets have more
+    // than one tile to count over, and keep the radix sort.
     constexpr uint32_t kRankKeys   = 64; // keys per block
     constexpr uint32_t kRankSlices = 16;
 

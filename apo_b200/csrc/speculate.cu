@@ -32,8 +32,9 @@ namespace apo2
 #define APO2_SPEC_MIN_BLOCKS 4
 #endif
     // Nodes one lane may visit before the search goes to a warp. The lane kernel lasts as long as its
-    // longest walk, some 1.9 us a node: of 128 / 256 / 512 nodes, 10k uniform sites 5.8 / 6.2 / 6.5 ms,
-    // 1M log-normal cloud 321 / 318 / 318 ms.
+    // longest walk, some 1.9 us a node, which is what counts for few sites; many are better off with longer
+    // walks. All edge-search kernels, of 128 / 160 / 256 nodes: 1,000 uniform sites 1.55 / 1.61 / 1.87 ms,
+    // 10,000 2.8 / 2.9 / 3.3, 61k protein 14.5 / 14.4 / 14.9, 1M protein 127 / 121 / 119, 1M log-normal 198 / 185 / 176.
     constexpr uint32_t kLaneBudget    = APO2_SPEC_LANE_BUDGET;
     constexpr uint32_t kHeavyBlock    = 128;
     constexpr uint32_t kHeavyStack    = 3072; // shared node stack per warp of the cooperative walk
@@ -47,19 +48,11 @@ namespace apo2
     // is long FP64 code, and run by one or two lanes at a time it held the warp for most
     // of its time.
     constexpr uint32_t kRefillAt = APO2_SPEC_REFILL_AT;
-#ifndef APO2_SPEC_STEPS
-#define APO2_SPEC_STEPS 16
-#endif
-    constexpr uint32_t kSpecSteps = APO2_SPEC_STEPS; // nodes of every walk between two votes
-#ifndef APO2_BISECTOR_REFILL_AT
-#define APO2_BISECTOR_REFILL_AT 24
-#endif
-#ifndef APO2_BISECTOR_STEPS
-#define APO2_BISECTOR_STEPS 8
-#endif
+    constexpr uint32_t kSpecSteps = 16; // nodes of every walk between two votes
     // the same for the bisectors, whose set-up is short, and the nodes a walk takes between two votes
-    constexpr uint32_t kBisectorRefillAt = APO2_BISECTOR_REFILL_AT;
-    constexpr uint32_t kBisectorSteps    = APO2_BISECTOR_STEPS;
+    // (nodes / idle lanes, 1M protein packing: 4 / 16 5.5 ms, 8 / 8 5.7, 8 / 16 5.4, 8 / 24 5.0, 16 / 16 5.2)
+    constexpr uint32_t kBisectorRefillAt = 24;
+    constexpr uint32_t kBisectorSteps    = 8;
 
     __device__ __forceinline__ uint32_t lane_of() { return threadIdx.x & 31; }
 
@@ -307,12 +300,9 @@ namespace apo2
         settle_edge( c, s, open );
     }
 
-    // The walk is bound by the node steps (two boxes against three balls and two planes, 50 to 90
+    // The walk is bound by the node steps (two boxes against three balls and three planes, some hundred
     // nodes an edge); the balls of the arc and the planes replaced the ball around c_i, most of whose
-    // leaves went through a quadrisector solve each. First round's launches, 1M log-normal cloud:
-    // k_edge_speculate 245 -> 102 ms, k_edge_heavy_sub 111 -> 11, k_edge_heavy 20 -> 4; 1M-site protein
-    // packing 117 -> 74, 18.5 -> 8.1, 7.8 -> 3.3 ms; 46^3 lattice 6.6 -> 7.6 ms (equal radii: there
-    // the planes let little in before, and the set-up grew).
+    // leaves went through a quadrisector solve each.
     //
     // May the box hold a contributor? Without an arc, also the reference's own test for entering it
     // (algorithm.inl:642-667: the box meets the bounding sphere and, for a hyperbolic edge, the
@@ -423,9 +413,11 @@ namespace apo2
     // three balls, read by all lanes at once, where a walk of its own took 50 to 90 nodes of two boxes
     // each, on lanes that part at every node. Cells with more surroundings than the list holds (hull
     // cells) keep their items for k_edge_speculate, edges that reach past the list go to a warp of
-    // their own (k_edge_heavy). All edge-search kernels of a build: 1M log-normal cloud 124 -> 103 ms,
-    // 46^3 lattice 8.2 -> 6.2 ms, 100k uniform 14.0 -> 9 ms, 10k uniform 1.9 -> 1.8 ms, 1M-site protein
-    // packing 87 -> 86 ms.
+    // their own (k_edge_heavy). The set-up of an edge is straight double-precision code, run by 16 warps at 16
+    // places of it: the kernel's size decides whether it stays in the instruction cache (per issue of a warp, 2.9
+    // cycles of waiting for instructions at 93 KB of code, 8.4 at 104; it is 96 now). All edge-search kernels of a build, against searches bounded by one ball and
+    // a walk per edge: 1M log-normal cloud 387 -> 185 ms, 1M-site protein packing 146 -> 121, 100k uniform
+    // 27 -> 16, 46^3 lattice 6.7 -> 6.8.
     __global__ void __launch_bounds__( kCellBlock, 4 ) k_edge_cells( CellContext c, const uint32_t * __restrict__ tasks,
                                                                      const uint32_t * __restrict__ task_count, SpecBuffers b )
     {
@@ -1109,10 +1101,10 @@ namespace apo2
     size_t spec_bytes( uint32_t n )
     {
         auto a = []( size_t x ) { return ( x + 255 ) & ~size_t( 255 ); };
-        return a( 4 * size_t( n ) * kNbrCap ) + a( 4 * size_t( n ) ) * 4 + a( 4 * size_t( n ) ) + a( 16 ) * 3
-               + a( 4 * output_scan_scratch_words( n ) ) + a( sizeof( uint2 ) * heavy_capacity( n ) ) + a( 16 ) * 2
-               + a( 4 * size_t( n ) * kMaybeWords ) + a( sizeof( uint2 ) * sub_capacity( n ) ) + a( 16 ) * 2
-               + a( sizeof( EdgeSearch ) * split_capacity( n ) ) + a( 16 );
+        return a( 4 * size_t( n ) * kNbrCap ) + a( 4 * size_t( n ) ) * 5 + a( 16 )
+               + a( 4 * output_scan_scratch_words( n ) ) + a( sizeof( uint2 ) * heavy_capacity( n ) )
+               + a( 4 * size_t( n ) * kMaybeWords ) + a( sizeof( uint2 ) * sub_capacity( n ) )
+               + a( sizeof( EdgeSearch ) * split_capacity( n ) );
     }
 
     void spec_carve( SpecBuffers & b, void * base, uint32_t n )
@@ -1134,29 +1126,15 @@ namespace apo2
         p += a( 4 * size_t( n ) );
         b.item_total = reinterpret_cast<uint64_t *>( p );
         p += a( 16 );
-        b.item_counter = reinterpret_cast<uint64_t *>( p );
-        p += a( 16 );
-        b.exact_count = reinterpret_cast<uint32_t *>( p );
-        p += a( 16 );
         b.scan_sums = reinterpret_cast<uint32_t *>( p );
         p += a( 4 * output_scan_scratch_words( n ) );
         b.heavy = reinterpret_cast<uint2 *>( p );
         p += a( sizeof( uint2 ) * heavy_capacity( n ) );
-        b.heavy_count = reinterpret_cast<uint32_t *>( p );
-        p += a( 16 );
-        b.heavy_next = reinterpret_cast<uint32_t *>( p );
-        p += a( 16 );
         b.maybe_bits = reinterpret_cast<uint32_t *>( p );
         p += a( 4 * size_t( n ) * kMaybeWords );
         b.sub = reinterpret_cast<uint2 *>( p );
         p += a( sizeof( uint2 ) * sub_capacity( n ) );
-        b.sub_count = reinterpret_cast<uint32_t *>( p );
-        p += a( 16 );
-        b.sub_next  = reinterpret_cast<uint32_t *>( p );
-        p += a( 16 );
-        b.splits = p;
-        p += a( sizeof( EdgeSearch ) * split_capacity( n ) );
-        b.split_count = reinterpret_cast<uint32_t *>( p );
+        b.splits      = p;
         b.split_cap   = uint32_t( split_capacity( n ) );
         b.sub_cap   = uint32_t( sub_capacity( n ) );
         b.heavy_cap = uint32_t( heavy_capacity( n ) );
