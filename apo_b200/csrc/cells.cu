@@ -1806,7 +1806,7 @@ namespace apo2
                     OpenEnds   open;
                     reach = edge_reach( c, si, sk, sl, hyperbola, ends, bounded, wmax, bsph, open );
                     close_ends( c, si, k, l, ends, sites_of( w ), open, reach );
-                    settle( reach, open );
+                    settle( c, reach, open );
                 }
 
                 // proven free of contributors on this very cell state

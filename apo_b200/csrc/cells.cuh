@@ -738,7 +738,9 @@ namespace apo2
         const float margin = 1e-5f * ( around.w + fabsf( around.x ) + fabsf( around.y ) + fabsf( around.z ) );
         if ( around.w + margin < reach.limit.w )
             reach.limit = make_float4( around.x, around.y, around.z, around.w + margin );
-        reach.limit.w += float( c.scene->rmax - rmin ) + low;
+        else
+            reach.limit.w += float( c.scene->rmax - rmin );
+        reach.limit.w += low;
         reach.margin    = 1e-5f * ( reach.limit.w + fabsf( reach.limit.x ) + fabsf( reach.limit.y ) + fabsf( reach.limit.z ) );
         reach.diameter  = 2.f * fmaxf( 0.f, float( rmin ) );
         reach.below     = hyperbola && rmin >= 0.0;
@@ -751,7 +753,7 @@ namespace apo2
         return reach;
     }
     // Once its open ends have been looked at: an arc with one left is searched in the ball.
-    __device__ __forceinline__ void settle( EdgeReach & reach, const OpenEnds & open )
+    __device__ __forceinline__ void settle( const CellContext & c, EdgeReach & reach, const OpenEnds & open )
     {
         if ( reach.kind == kReachBall || open.mask )
         {
@@ -762,8 +764,9 @@ namespace apo2
             reach.far       = 1.f;
         }
         // a root of radius w touches the plane to L^2 / 2w at a distance of L, at most 2.5 times the
-        // limit's radius
-        reach.slab[ 0 ] = reach.slab[ 1 ] = 3.2f / reach.far * reach.limit.w * reach.limit.w + reach.margin;
+        // limit's radius and that of a site
+        const float span = reach.limit.w + fmaxf( 0.f, float( c.scene->rmax ) );
+        reach.slab[ 0 ]  = reach.slab[ 1 ] = 3.2f / reach.far * span * span + reach.margin;
     }
 
     // An apex (trisector root in the plane of the centres) counts unless a neighbour other

@@ -269,7 +269,7 @@ namespace apo2
     __device__ __forceinline__ void settle_edge( const CellContext & c, EdgeSearch & s, const OpenEnds & open )
     {
         const float4 fsi = to_float( s.si );
-        settle( s.reach, open );
+        settle( c, s.reach, open );
         if ( s.reach.kind == kReachArcPlanes )
         {
             bool open1 = true, open2 = true;
@@ -464,7 +464,7 @@ namespace apo2
                 __syncwarp();
                 close_ends_together( c, si, s.k, s.l, ends, SiteSequence { nbr, known, 0u }, loose, s.reach );
                 if ( open )
-                    settle( s.reach, loose );
+                    settle( c, s.reach, loose );
                 if ( open && !s.covered )
                 {
                     const uint32_t slot = atomicAdd( b.heavy_count, 1u );
