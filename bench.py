@@ -51,13 +51,13 @@ PEAKS_FALLBACK = {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0}
 C_QUAD = 216
 C_TEST = 11
 
-# DRAM bytes (read + write) per site of one launch, by kernel, from ncu captures of the kernel's first
-# launch on the log-normal cloud of 300,000 sites at the evaluation density, scaled by the sites
-# processed. The other kernels have no capture.
-TRAFFIC_BYTES_PER_SITE = {"k_vertex_validation": (1643.8, "300k log-normal capture"),
-                          "k_edge_cells": (1430.7, "300k log-normal capture"),
-                          "k_cells": (528.8, "300k log-normal capture"),
-                          "k_edge_speculate": (134.4, "300k log-normal capture")}
+# DRAM bytes (read + write) of each kernel's first launch, plain form, log-normal cloud of 300,000 sites at the
+# evaluation density (profiles/dram_logn300k.md). They hold for that workload only: its nodes and sites fit
+# the L2, and from 400,000 cells the vertex validation's first launch is another instantiation.
+TRAFFIC_SITES = 300000
+TRAFFIC_BYTES = {"k_cells": 159953152, "k_vertex_validation": 489802240, "k_edge_cells": 1163659008,
+                 "k_edge_speculate": 114850816, "k_edge_heavy": 117668096, "k_edge_heavy_sub": 32336384,
+                 "k_edge_validation": 116278016}
 
 
 def measure_fp64_peak(device) -> float:
@@ -498,10 +498,11 @@ def run_ours(args, world, rank, local):
     roofline = {
         "bound": "hbm", "kernel": dom_name, "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
         "frac": achieved / peaks["hbm_gbs"],
-        "traffic": (TRAFFIC_BYTES_PER_SITE[dom_name][0] * n if dom_name in TRAFFIC_BYTES_PER_SITE else None),
-        "traffic_note": ("ncu dram__bytes_read.sum + dram__bytes_write.sum of the kernel's first (longest) launch, "
-                         f"{TRAFFIC_BYTES_PER_SITE[dom_name][1]}, scaled by sites" if dom_name in TRAFFIC_BYTES_PER_SITE
-                         else "no capture of this kernel"), "peak_kind": peaks_kind,
+        "traffic": (TRAFFIC_BYTES.get(dom_name) if (n, args.form) == (TRAFFIC_SITES, "plain") else None),
+        "traffic_note": "ncu dram__bytes_read.sum + dram__bytes_write.sum of the kernel's first (longest) launch",
+        "traffic_capture": {"sites": TRAFFIC_SITES, "form": "plain", "bytes": TRAFFIC_BYTES.get(dom_name),
+                            "file": "profiles/dram_logn300k.md"},
+        "peak_kind": peaks_kind,
         "kernel_share": dom_ms / total_ms, "kernel_avg_launch_ms": dom_avg_ms, "kernel_launches": dom_count,
         "launch": "the kernel's longest launch (first validation round)", "launch_ms": dom_max_ms,
         "algorithmic_bytes_per_launch": dom_bytes_per_launch,
