@@ -42,3 +42,20 @@ def test_stores_match_the_oracle(kind, n, seed, precision):
         assert np.array_equal(algo.debug_array(name), ref[name]), name
     assert np.array_equal(algo.toHost().verticesId, ref["out_vertices_id"])
     algo.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_searches_handed_to_a_warp(precision):
+    """Long searches (edges of hull cells whose bounds cover much of the cloud): set up again by the warp
+    that they go to, whichever way it would decide whether the security radius covers them."""
+    import apo_b200
+    from apo_b200 import generators
+    from oracle import oracle
+    sites = generators.uniform_random(3000, 66.9, 0.5, 2.0, 5)
+    ref = oracle.build(sites)
+    assert ref["flags"] == 0
+    algo = apo_b200.AlgorithmGPU(sites, precision=precision)
+    algo.build()
+    for name in ("indices", "status", "vertex_nb", "edge_nb", "vertices", "edges"):
+        assert np.array_equal(algo.debug_array(name), ref[name]), name
+    algo.close()
