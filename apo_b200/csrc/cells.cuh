@@ -424,7 +424,7 @@ namespace apo2
 
     __device__ __forceinline__ float4 neighbour( const CellContext & c, uint32_t u ) { return u < c.n ? c.sites_f[ u ] : to_float( c.sites[ u ] ); }
 
-    // Where the conflict of an end's third site ends again, further out: the point and its radius, what the
+    // Shortly before the conflict of an end's third site ends again, further out: the point and its radius, what the
     // curve goes on to (a hyperbola to infinity, in a direction; an ellipse to a point half-way round to
     // the other end, with its radius), and the least radius on the way.
     struct OpenEnds
@@ -581,10 +581,12 @@ namespace apo2
                 far = fminf( far, slope * root );
                 continue;
             }
-            // it ends at the site's other root: another neighbour has to take over there
+            // it ends at the site's other root: another neighbour has to take over before, a fiftieth of the way,
+            // which is more than the rounding of that root's place
             const float q = f.y / f.x, w = 1.f - fal * q * q;
-            const float s = -2.f * q * ( fal * ( x.x + q * x.y ) - fbe ) / w - x.y, rho = x.x + q * ( x.y - s );
-            if ( !( f.x < 0.f && w > 1e-3f && out * ( s - x.y ) > 0.f && fal * rho > fbe && rho < float( kFarRoot ) ) )
+            const float last = -2.f * q * ( fal * ( x.x + q * x.y ) - fbe ) / w - x.y;
+            const float s    = last - .02f * ( last - x.y ), rho = ( fbe + sqrtf( fmaxf( fbe * fbe + fal * ( float( gamma ) + s * s ), 0.f ) ) ) / fal;
+            if ( !( f.x < 0.f && w > 1e-3f && out * ( last - x.y ) > 0.f && fal * ( x.x + q * ( x.y - last ) ) > fbe && rho < float( kFarRoot ) ) )
                 return false;
             open.add( a, fA + fB * rho + fn * s, rho - fi.w, fB + fn * ( out * root ), 0.f, least );
         }
@@ -596,7 +598,7 @@ namespace apo2
         else
         {
             // Half-way round, opposite the piece, each of the two has to hold, or another neighbour has to take
-            // over where it ends, at its other root: the end's mirror image in the gradient (all in the
+            // over before it ends, at its other root: the end's mirror image in the gradient (all in the
             // ellipse's unit circle)
             const float  low = frc - arf - fi.w;
             const float2 e0 = make_float2( float( c0.x ), float( c0.y ) ), e1 = make_float2( float( c1.x ), float( c1.y ) );
@@ -612,8 +614,10 @@ namespace apo2
                 const float2 v = make_float2( f.x * arf, f.y * fas );
                 if ( v.x * ( half.x - x.x ) + v.y * ( half.y - x.y ) > deep )
                     continue;
-                const float  m = 2.f * ( v.x * x.x + v.y * x.y ) / ( v.x * v.x + v.y * v.y );
-                const float2 y = make_float2( m * v.x - x.x, m * v.y - x.y );
+                const float  vv = v.x * v.x + v.y * v.y, m = 2.f * ( v.x * x.x + v.y * x.y ) / vv + .02f * rsqrtf( vv );
+                const float2 z  = make_float2( m * v.x - x.x, m * v.y - x.y );
+                const float  iz = rsqrtf( z.x * z.x + z.y * z.y );
+                const float2 y  = make_float2( iz * z.x, iz * z.y );
                 open.add( a, fA + fB * ( frc + arf * y.x ) + fn * ( fas * y.y ), frc + arf * y.x - fi.w,
                           fA + fB * ( frc + arf * half.x ) + fn * ( fas * half.y ), frc + arf * half.x - fi.w, low );
             }
